@@ -39,3 +39,46 @@ def test_sampling_at_every_share_of_a_warp(eng, orc, k):
             want, state = orc.sample_from_topk(idx[m], val[m], float(np.float32(t)), k,
                                                float(np.float32(p)), int(state0[m]))
             assert (got[m], int(new[m])) == (want, state), (m, t, p)
+
+
+def _quantize_equal(eng, orc, wb):
+    import torch
+    packed, scale = eng.quantize_w4a16(to_dev(wb, torch.bfloat16))
+    want_p, want_s = orc.quantize_w4a16(wb)
+    assert np.array_equal(from_dev(packed), want_p)
+    assert np.array_equal(from_dev(scale).view(np.uint16), want_s.view(np.uint16))
+
+
+def test_quantizer_on_every_pair_of_significands(eng, orc):
+    """The group maximum takes each of the 128 bf16 significands, the other values of its
+    groups every bf16 of the same and the next 13 lower exponents, of either sign: each
+    rounding boundary and each exact tie there is (14 |w| an odd multiple of the maximum)."""
+    rest = np.arange((127 - 13) << 7, (127 << 7) + 128, dtype=np.uint16)
+    groups = []
+    for a in range(128):
+        top = (127 << 7) | a
+        w = rest[rest <= top]
+        w = np.concatenate([w, w | 0x8000])
+        w = np.concatenate([w, np.zeros(-w.size % 127, np.uint16)]).reshape(-1, 127)
+        groups.append(np.concatenate([np.full((w.shape[0], 1), top, np.uint16), w], axis=1))
+    wb = np.concatenate(groups)
+    n = wb.shape[0] // 8
+    _quantize_equal(eng, orc, np.ascontiguousarray(wb[:n * 8].reshape(n, 1024)))
+
+
+@pytest.mark.parametrize("exponent", [1, 20, 34, 36, 38, 40, 127, 216, 218, 220, 222, 250, 254])
+def test_quantizer_over_the_exponents(eng, orc, exponent):
+    """Scales either side of the range in which the packed arithmetic is exact, down to
+    subnormal ones and up to the largest bf16."""
+    rng = np.random.default_rng(BASE_SEED + exponent)
+    e = np.clip(exponent - rng.integers(0, 10, (64, 256)), 0, 254).astype(np.uint16)
+    wb = (e << 7) | rng.integers(0, 128, e.shape, dtype=np.uint16) | (rng.integers(0, 2, e.shape, dtype=np.uint16) << 15)
+    _quantize_equal(eng, orc, wb.astype(np.uint16))
+
+
+@pytest.mark.parametrize("N,K", [(1, 128), (1, 1920), (1, 2048), (1, 2176), (15, 128), (17, 128), (129, 384),
+                                 (4737, 1024), (18944, 128), (18945, 128)])
+def test_quantizer_group_counts(eng, orc, N, K):
+    """Group counts around a warp's sixteen and around a whole grid of them."""
+    rng = np.random.default_rng(BASE_SEED + N)
+    _quantize_equal(eng, orc, orc.f32_to_bf16_bits((rng.standard_normal((N, K)) * 0.02).astype(np.float32)))
