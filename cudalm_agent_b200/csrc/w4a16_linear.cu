@@ -19,12 +19,16 @@ int run_tc_with_pick(const cudalm_b200_linear& l, const PickTail& pick, cudaStre
 int run_tc_extra(const cudalm_b200_linear& l, const std::uint8_t* weight2,
                  const std::uint16_t* scales2, const std::uint16_t* residual, cudaStream_t stream);
 struct TcGroup;
+bool rows_eligible(const cudalm_b200_linear& l);
+int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight2, const std::uint16_t* scales2,
+             const std::uint16_t* residual, cudaStream_t stream);
 int tc_group_create(const cudalm_b200_linear* ls, int count, TcGroup** out);
 int tc_group_run(const TcGroup* g, cudaStream_t stream);
 void tc_group_destroy(TcGroup* g);
 // Smallest M that takes the tensor-memory kernel (runtime knob; see
 // cudalm_b200_set_tensor_path_min_rows).
 std::atomic<int> g_tc_min_rows{17};
+constexpr int kTcMaxRows = 64;  // most activation rows of the kernel in w4a16_tc.cu
 // lean kernel for single calls of a few megabytes (w4a16_direct.cu)
 bool direct_eligible(const cudalm_b200_linear& l, const std::uint8_t* weight2);
 long long direct_weight_bytes(const cudalm_b200_linear& l, bool pair);
@@ -381,19 +385,9 @@ int run_single(cudalm_b200_linear l, cudaStream_t stream) {
       direct_weight_bytes(l, false) <= g_direct_max_bytes.load(std::memory_order_relaxed))
     return run_direct(&l, 1, nullptr, nullptr, nullptr, stream);
   if (l.M >= g_tc_min_rows.load(std::memory_order_relaxed)) {
-    // passes of up to 64 rows on the tensor-memory kernel
-    cudalm_b200_linear probe = l;
-    probe.M = l.M < 64 ? l.M : 64;
-    if (tc_eligible(probe)) {
-      for (int m0 = 0; m0 < l.M; m0 += 64) {
-        cudalm_b200_linear part = l;
-        part.M = (l.M - m0 < 64) ? (l.M - m0) : 64;
-        part.x = l.x + static_cast<std::size_t>(m0) * l.K;
-        part.y = l.y + static_cast<std::size_t>(m0) * l.N;
-        if (int rc = run_tc(&part, 1, stream)) return rc;
-      }
-      return CUDALM_B200_OK;
-    }
+    // the tensor-memory kernels: one for up to 64 rows, one for any number above
+    if (l.M <= kTcMaxRows && tc_eligible(l)) return run_tc(&l, 1, stream);
+    if (l.M > kTcMaxRows && rows_eligible(l)) return run_rows(&l, 1, nullptr, nullptr, nullptr, stream);
   }
   if (!stream_eligible(l)) return run_fallback(l, stream);
   const int per_pass = max_rows_per_pass(l.K);
@@ -430,22 +424,13 @@ int run_extra(cudalm_b200_linear l, const LinearExtra& ex, cudaStream_t stream) 
     return run_direct(&l, 1, w2, s2, rs, stream);
   }
   if (l.M >= g_tc_min_rows.load(std::memory_order_relaxed)) {
-    // passes of up to 64 rows on the tensor-memory kernel, when it takes the call
-    bool done = true;
-    for (int m0 = 0; m0 < l.M && done; m0 += 64) {
-      cudalm_b200_linear part = l;
-      part.M = (l.M - m0 < 64) ? (l.M - m0) : 64;
-      part.x = l.x + static_cast<std::size_t>(m0) * l.K;
-      part.y = l.y + static_cast<std::size_t>(m0) * l.N;
-      const int rc = tc_eligible(part)
-                         ? run_tc_extra(part, ex.weight2, ex.scales2,
-                                        ex.residual ? ex.residual + static_cast<std::size_t>(m0) * l.N : nullptr,
-                                        stream)
-                         : CUDALM_B200_ERR_UNSUPPORTED;
-      if (rc == CUDALM_B200_ERR_UNSUPPORTED && m0 == 0) done = false;  // streaming passes instead
-      else if (rc != CUDALM_B200_OK) return rc;
-    }
-    if (done) return CUDALM_B200_OK;
+    // the tensor-memory kernels, when they take the call
+    int rc = CUDALM_B200_ERR_UNSUPPORTED;
+    if (l.M > kTcMaxRows)
+      rc = run_rows(&l, 1, ex.weight2, ex.scales2, ex.residual, stream);
+    else if (tc_eligible(l))
+      rc = run_tc_extra(l, ex.weight2, ex.scales2, ex.residual, stream);
+    if (rc != CUDALM_B200_ERR_UNSUPPORTED) return rc;
   }
   int per_pass = stream_eligible(l) && (!pair || aligned_to(ex.weight2, 16)) ? max_rows_per_pass(l.K) : 0;
   if (per_pass > 16) per_pass = 16;
@@ -579,6 +564,9 @@ int cudalm_b200_linear_multi(const cudalm_b200_linear* linears, int count, void*
     bool all_tc = true;
     for (int i = 0; i < count; ++i) all_tc &= tc_eligible(linears[i]);
     if (all_tc) return run_tc(linears, count, st);
+    bool all_rows = mmax > kTcMaxRows;
+    for (int i = 0; i < count; ++i) all_rows &= rows_eligible(linears[i]);
+    if (all_rows) return run_rows(linears, count, nullptr, nullptr, nullptr, st);
   }
   Plan pl;
   if (!all_stream || mmax > CUDALM_B200_MAX_GROUP_M || !make_plan(kmax, mmax, &pl)) {
@@ -610,9 +598,9 @@ int cudalm_b200_gate_up_bf16(const uint8_t* gate_weight, const uint16_t* gate_sc
   // rows of x beyond what one launch holds go in further passes
   int per_pass = (K > 0 && K % 128 == 0 && K <= kMaxStreamK) ? max_rows_per_pass(K) : 0;
   if (per_pass == 0) per_pass = M;
-  // batched rows go to the tensor-memory kernel in passes of 64 (linear_multi falls
-  // back to the streaming kernel, in its own passes, when that kernel does not take them)
-  if (M >= g_tc_min_rows.load(std::memory_order_relaxed)) per_pass = 64;
+  // batched rows go to the tensor-memory kernels in one launch (linear_multi falls back
+  // to the streaming kernel, in its own passes, when they do not take them)
+  if (M >= g_tc_min_rows.load(std::memory_order_relaxed)) per_pass = M;
   for (int m0 = 0; m0 < M; m0 += per_pass) {
     const int mm = (M - m0 < per_pass) ? (M - m0) : per_pass;
     cudalm_b200_linear two[2] = {

@@ -1,0 +1,594 @@
+// Many activation rows (a prompt: more than 64) on the fifth-generation tensor cores.
+//
+// One CTA per SM works on units of 128 weight rows x NT activation rows of one projection
+// (NT = 256, 128 or 64).  The weight rows are the M dimension of the MMA (A, in tensor
+// memory), the activation rows its N dimension (B, in shared memory).  Per quantisation
+// group of 128 k:
+//
+//   * 128 "dequantising" threads, one per weight row, turn the row's 64 packed bytes into
+//     exact bf16 integers and write them to tensor memory (tcgen05.st).  Two sets of 128
+//     take alternate groups;
+//   * an issuing thread runs the group's eight K=16 MMAs into a fresh fp32 accumulator
+//     slot (two issuers with a slot each at NT = 256);
+//   * 256 "fold" threads read the slot back and add scale * sum to the unit's running
+//     sums in registers, NT / 2 per thread, two to an instruction (fma.rn.f32x2).
+//
+// The group's scale multiplies its fp32 sum, as in the kernel for up to 64 rows: folding
+// it into the bf16 operand would round it away (an fp16 scale times a 4-bit integer has 14
+// significant bits).  Products are exact and sums are fp32.
+//
+// Work runs along three rings: packed weights (shared memory, two groups per stage),
+// activations (shared memory, one group per stage) and A buffers / accumulator slots
+// (tensor memory).
+//
+// Every wait is bounded; a wait that runs out raises a CTA-wide abort flag, the kernel
+// stores ERR_TIMEOUT in the status word, frees its tensor memory and returns.
+#include <cuda.h>
+
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+#include "common.cuh"
+#include "tcgen05.cuh"
+
+namespace cb200 {
+namespace {
+
+enum : int { kRowsPlain = 0, kRowsPair = 1, kRowsResidual = 2 };
+
+struct alignas(64) RowsDesc {
+  CUtensorMap tmap;   // weights as uint32 [N][K/8], box 128 rows (a pair: 64) x 32 words
+  CUtensorMap tmap2;  // kRowsPair: the second (up) matrix
+  CUtensorMap xmap;   // activations as bf16 [M][K], box NT rows x 64 values
+  const std::uint16_t* S;
+  const std::uint16_t* S2;   // kRowsPair: scales of the second matrix
+  const std::uint16_t* res;  // kRowsResidual: residual [M][N]; may be y
+  std::uint16_t* y;
+  int N, K, M;
+  int mode;
+  int tok_tiles;   // unit = weight tile * tok_tiles + activation tile
+  int unit_begin;  // first unit of this projection in the launch
+  int unit_end;
+  int cost_begin;  // groups before this projection
+};
+
+struct RowsParams {
+  RowsDesc d[CUDALM_B200_MAX_INLINE_LINEARS];
+  int n_desc;
+  int total_units;
+  int total_cost;
+  int* status;
+};
+
+// Register shares (of the 640 x 96 the CTA is launched with; 256 fold, 256 dequantising
+// and 128 other threads): 256 x 176 + 256 x 48 + 128 x 32 = 61440 where a fold thread keeps
+// 128 sums, 256 x 136 + 256 x 72 + 128 x 64 = 61440 otherwise.
+template <int NT>
+struct RowsCfg {
+  static constexpr int kSub = NT == 256 ? 2 : 1;         // MMAs along N per K=16 step (N <= 128 each)
+  static constexpr int kSlot = NT / kSub;                // columns of an accumulator slot
+  static constexpr int kAcc = NT / 2;                    // running sums per fold thread
+  static constexpr int kD = NT == 256 ? 3 : (NT == 128 ? 2 : 4);  // accumulator slots
+  // Barrier pairs per issuer.  NT = 256: the three slots go round over both issuers, so one
+  // of them can hold all three; four pairs keep it from lapping a barrier.
+  static constexpr int kDB = NT == 256 ? 4 : kD;
+  static constexpr int kA = NT == 256 ? 2 : 4;           // A buffers of 64 columns
+  static constexpr int kW = NT == 256 ? 2 : (NT == 128 ? 4 : 6);  // weight stages, 16 KB
+  static constexpr int kB = NT == 256 ? 3 : (NT == 128 ? 4 : 6);  // activation stages
+  static constexpr int kBoxBytes = NT * 128;             // NT rows x 64 values
+  static constexpr int kBBytes = 2 * kBoxBytes;
+  static constexpr int kRegFold = NT == 256 ? 176 : 136;
+  static constexpr int kRegDequant = NT == 256 ? 48 : 72;
+  static constexpr int kRegOther = NT == 256 ? 32 : 64;
+  static_assert(kD * kSlot + kA * 64 <= 512, "tensor memory");
+};
+constexpr int kRowsWBytes = kTcRowsPerTile * 128;
+constexpr int kRowsHeaderBytes = 1024;
+template <int NT>
+constexpr int rows_smem_bytes() {
+  return 1024 + kRowsHeaderBytes + RowsCfg<NT>::kW * kRowsWBytes + RowsCfg<NT>::kB * RowsCfg<NT>::kBBytes;
+}
+
+// Warp roles: 0..3 and 4..7 dequantise even / odd groups, 8..11 and 12..15 fold (each half
+// of the activation rows), 16 copies weights, 18 activations, 17 and 19 issue MMAs.
+constexpr int kRowsThreads = 640;
+constexpr int kRowsFoldWarp0 = 8;
+constexpr int kRowsWeightWarp = 16;
+constexpr int kRowsIssueWarp = 17;  // second issuer: + 2
+constexpr int kRowsActWarp = 18;
+
+struct RowsSmem {
+  std::uint64_t w_full[6], w_empty[6];
+  std::uint64_t b_full[6], b_empty[6];
+  std::uint64_t a_full[4], a_empty[4];
+  std::uint64_t d_full[2][4], d_free[2][4];  // [issuer][slot use]
+  std::uint32_t tmem_base;
+  int abort_flag;
+};
+static_assert(sizeof(RowsSmem) <= kRowsHeaderBytes, "barrier block too large");
+
+// A position in a ring of n stages and the parity of the phase it is in.
+struct Ring {
+  int i = 0;
+  std::uint32_t phase = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++i == n) {
+      i = 0;
+      phase ^= 1u;
+    }
+  }
+};
+
+// acc += {s, s} * {d0, d1}; volatile, so that it stays behind the wait for the tensor-memory
+// load that d0 and d1 come from.
+__device__ __forceinline__ void fma_f32x2(unsigned long long& acc, std::uint32_t d0, std::uint32_t d1,
+                                          unsigned long long s2) {
+  asm volatile("{\n\t.reg .b64 p;\n\tmov.b64 p, {%1, %2};\n\tfma.rn.f32x2 %0, p, %3, %0;\n\t}"
+               : "+l"(acc)
+               : "r"(d0), "r"(d1), "l"(s2));
+}
+__device__ __forceinline__ float lo_f(unsigned long long v) {
+  return __uint_as_float(static_cast<std::uint32_t>(v));
+}
+__device__ __forceinline__ float hi_f(unsigned long long v) {
+  return __uint_as_float(static_cast<std::uint32_t>(v >> 32));
+}
+
+template <int NT, bool EXTRA>
+__global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __grid_constant__ RowsParams p) {
+  using C = RowsCfg<NT>;
+  extern __shared__ __align__(1024) std::uint8_t smem_raw[];
+  // the swizzled TMA destinations need 1024-byte alignment; the launch adds the slack
+  std::uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  RowsSmem* sm = reinterpret_cast<RowsSmem*>(smem);
+  std::uint8_t* wst = smem + kRowsHeaderBytes;
+  std::uint8_t* bst = wst + C::kW * kRowsWBytes;
+  volatile int* abort_flag = &sm->abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int i = 0; i < C::kW; ++i) {
+      mbar_init(&sm->w_full[i], 1);
+      mbar_init(&sm->w_empty[i], 8);  // once per dequantising warp
+    }
+    for (int i = 0; i < C::kB; ++i) {
+      mbar_init(&sm->b_full[i], 1);
+      mbar_init(&sm->b_empty[i], C::kSub);
+    }
+    for (int i = 0; i < C::kA; ++i) {
+      mbar_init(&sm->a_full[i], 4);
+      mbar_init(&sm->a_empty[i], C::kSub);
+    }
+    for (int h = 0; h < C::kSub; ++h)
+      for (int i = 0; i < C::kDB; ++i) {
+        mbar_init(&sm->d_full[h][i], 1);
+        mbar_init(&sm->d_free[h][i], C::kSub == 2 ? 4 : 8);
+      }
+    sm->abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 0) tmem_alloc(&sm->tmem_base, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const std::uint32_t tmem_d = sm->tmem_base;
+  const std::uint32_t tmem_a = tmem_d + C::kD * C::kSlot;
+
+  // This CTA's contiguous range of units: an equal share of the groups.
+  auto unit_at = [&](long long cost) -> int {
+    if (cost >= p.total_cost) return p.total_units;
+    int d = p.n_desc - 1;
+    while (d > 0 && p.d[d].cost_begin > cost) --d;
+    const int per = p.d[d].K >> 7;
+    return p.d[d].unit_begin + static_cast<int>((cost - p.d[d].cost_begin + per - 1) / per);
+  };
+  const int u_lo = unit_at(static_cast<long long>(blockIdx.x) * p.total_cost / gridDim.x);
+  const int u_hi = unit_at(static_cast<long long>(blockIdx.x + 1) * p.total_cost / gridDim.x);
+  int di = 0;  // projection of the current unit
+  auto seek = [&](int u) {
+    while (u >= p.d[di].unit_end) ++di;
+  };
+
+  // Programmatic dependent launch: only the weight copies (weights are nobody's output)
+  // may run before the preceding kernel has completed.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (warp != kRowsWeightWarp) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  if (warp >= kRowsWeightWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegOther) : "memory");
+    if (warp == kRowsWeightWarp) {
+      if (lane == 0) {
+        // ---------------- packed weights ----------------
+        Ring w;
+        bool first_round = true, ok = true;
+        for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
+          seek(u);
+          const RowsDesc& L = p.d[di];
+          const bool pair = EXTRA && L.mode == kRowsPair;
+          const int j = (u - L.unit_begin) / L.tok_tiles;
+          const int stages = ((L.K >> 7) + 1) >> 1;
+          for (int c = 0; c < stages; ++c) {
+            if (!first_round && !tc_wait(&sm->w_empty[w.i], w.phase ^ 1u, abort_flag)) {
+              ok = false;
+              break;
+            }
+            std::uint8_t* st = wst + w.i * kRowsWBytes;
+            mbar_arrive_expect_tx(&sm->w_full[w.i], kRowsWBytes);
+            for (int m = 0; m < (pair ? 2 : 1); ++m) {
+              asm volatile(
+                  "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+                  " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(st + m * (kRowsWBytes / 2))),
+                  "l"(m ? &L.tmap2 : &L.tmap), "r"(c * 32), "r"(j * (pair ? 64 : 128)),
+                  "r"(smem_u32(&sm->w_full[w.i]))
+                  : "memory");
+            }
+            w.next(C::kW);
+            if (w.i == 0) first_round = false;
+          }
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+      }
+    } else if (warp == kRowsActWarp) {
+      if (lane == 0) {
+        // ---------------- activations ----------------
+        Ring b;
+        bool first_round = true, ok = true;
+        for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
+          seek(u);
+          const RowsDesc& L = p.d[di];
+          const int t = (u - L.unit_begin) % L.tok_tiles;
+          const int G = L.K >> 7;
+          for (int g = 0; g < G; ++g) {
+            if (!first_round && !tc_wait(&sm->b_empty[b.i], b.phase ^ 1u, abort_flag)) {
+              ok = false;
+              break;
+            }
+            std::uint8_t* st = bst + b.i * C::kBBytes;
+            // rows past M arrive as zeros
+            mbar_arrive_expect_tx(&sm->b_full[b.i], C::kBBytes);
+            for (int q = 0; q < 2; ++q) {
+              asm volatile(
+                  "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+                  " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(st + q * C::kBoxBytes)),
+                  "l"(&L.xmap), "r"(g * 128 + q * 64), "r"(t * NT), "r"(smem_u32(&sm->b_full[b.i]))
+                  : "memory");
+            }
+            b.next(C::kB);
+            if (b.i == 0) first_round = false;
+          }
+        }
+      }
+    } else if (warp == kRowsIssueWarp || C::kSub == 2) {
+      if (lane == 0) {
+        // ---------------- MMA issue ----------------
+        const int h = (warp - kRowsIssueWarp) >> 1;  // half of the activation rows (NT = 256)
+        const std::uint32_t desc_hi = static_cast<std::uint32_t>(tc_b_desc(0) >> 32);
+        const std::uint32_t desc_lo0 = static_cast<std::uint32_t>(tc_b_desc(0));
+        const std::uint32_t b0 = smem_u32(bst) + static_cast<std::uint32_t>(h) * 128u * 128u;
+        constexpr std::uint32_t kIdesc = tc_idesc(C::kSlot);
+        Ring a, b;
+        std::uint32_t git = 0;
+        int slot = h;  // NT = 256: slots go round over both halves, 2 git + h modulo 3
+        bool ok = true;
+        for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
+          seek(u);
+          const int G = p.d[di].K >> 7;
+          for (int g = 0; g < G; ++g, ++git) {
+            // The slot's previous sums have been read.  NT = 256: they were the other
+            // half's, three slot uses ago, i.e. of group git - 1 (h = 1) or git - 2 (h = 0);
+            // otherwise those of kD groups ago.
+            if (C::kSub == 2) {
+              const std::uint32_t back = h == 1 ? 1u : 2u;
+              if (git >= back)
+                ok = tc_wait(&sm->d_free[1 - h][(git - back) % C::kDB], ((git - back) / C::kDB) & 1u, abort_flag);
+            } else if (git >= C::kD) {
+              ok = tc_wait(&sm->d_free[0][git % C::kD], ((git / C::kD) - 1u) & 1u, abort_flag);
+            }
+            ok = ok && tc_wait(&sm->b_full[b.i], b.phase, abort_flag) &&
+                 tc_wait(&sm->a_full[a.i], a.phase, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const std::uint32_t b_addr = b0 + b.i * C::kBBytes;
+            tc_mma_group(tmem_d + slot * C::kSlot, tmem_a + a.i * 64,
+                         desc_lo0 | ((b_addr & 0x3FFFFu) >> 4), desc_hi, C::kBoxBytes >> 4, kIdesc);
+            tc_commit(&sm->d_full[h][git % C::kDB]);
+            tc_commit(&sm->a_empty[a.i]);
+            tc_commit(&sm->b_empty[b.i]);
+            a.next(C::kA);
+            b.next(C::kB);
+            slot += C::kSub;
+            if (slot >= C::kD) slot -= C::kD;
+          }
+        }
+      }
+    }
+  } else if (warp < kRowsFoldWarp0) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegDequant) : "memory");
+    // ---------------- dequantise: the A operand ----------------
+    const std::uint32_t set = warp >> 2;  // takes the groups of this parity
+    const int lrow = (warp & 3) * 32 + lane;
+    const std::uint32_t a_base = tmem_a + (static_cast<std::uint32_t>((warp & 3) * 32) << 16);
+    std::uint32_t git = 0;
+    Ring w;
+    bool alive = true;
+    for (int u = u_lo; u < u_hi && alive; ++u) {
+      seek(u);
+      const int G = p.d[di].K >> 7;
+      // a pair's rows alternate gate, up (64 rows of either matrix)
+      const bool pair = EXTRA && p.d[di].mode == kRowsPair;
+      const int srow = pair ? (lrow & 1) * 64 + (lrow >> 1) : lrow;
+      for (int g = 0; g < G; ++g, ++git) {
+        if ((g & 1) == 0) {
+          const bool ok = tc_wait(&sm->w_full[w.i], w.phase, abort_flag);
+          alive = __all_sync(0xffffffffu, ok);
+          if (!alive) break;
+        }
+        if ((git & 1u) == set) {
+          const std::uint32_t buf = git % C::kA, use = git / C::kA;
+          if (use >= 1) {
+            const bool ok = tc_wait(&sm->a_empty[buf], (use - 1u) & 1u, abort_flag);
+            alive = __all_sync(0xffffffffu, ok);
+            if (!alive) break;
+          }
+          tc_fence_after();
+          const std::uint8_t* rowp = wst + w.i * kRowsWBytes + srow * 128;
+          const std::uint32_t a_addr = a_base + buf * 64;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            std::uint32_t regs[16];
+            const uint4 v = lds128(rowp + (((4 * (g & 1) + q) ^ (srow & 7)) << 4));
+            dequant_word_natural(v.x, regs);
+            dequant_word_natural(v.y, regs + 4);
+            dequant_word_natural(v.z, regs + 8);
+            dequant_word_natural(v.w, regs + 12);
+            tmem_st16(a_addr + 16 * q, regs);
+          }
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm->a_full[buf]);
+        }
+        if ((g & 1) || g == G - 1) {
+          // both sets have seen the stage's `full` phase and taken their group (if any)
+          // out of it
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm->w_empty[w.i]);
+          w.next(C::kW);
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegFold) : "memory");
+    // ---------------- fold: acc += scale * sum ----------------
+    const int f = (warp - kRowsFoldWarp0) >> 2;  // half of the activation rows
+    const int h = C::kSub == 2 ? f : 0;
+    const int lrow = (warp & 3) * 32 + lane;
+    const std::uint32_t d_base = tmem_d + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) +
+                                 (C::kSub == 2 ? 0u : static_cast<std::uint32_t>(f) * C::kAcc);
+    std::uint32_t git = 0;
+    int slot = h;
+    bool alive = true;
+    for (int u = u_lo; u < u_hi && alive; ++u) {
+      seek(u);
+      const RowsDesc& L = p.d[di];
+      const int N = L.N, G = L.K >> 7;
+      const int j = (u - L.unit_begin) / L.tok_tiles, t = (u - L.unit_begin) - j * L.tok_tiles;
+      const bool pair = EXTRA && L.mode == kRowsPair;
+      const int row = pair ? j * 64 + (lrow >> 1) : j * 128 + lrow;
+      const bool row_ok = row < N;
+      const std::uint16_t* srow = ((pair && (lrow & 1)) ? L.S2 : L.S) + static_cast<std::size_t>(row_ok ? row : 0) * G;
+      unsigned long long acc[C::kAcc / 2];
+#pragma unroll
+      for (int n = 0; n < C::kAcc / 2; ++n) acc[n] = 0ull;
+      // the scale of the next group is fetched while this one's sums are awaited
+      std::uint16_t sc_bits = __ldg(srow);
+      for (int g = 0; g < G; ++g, ++git) {
+        const std::uint32_t sc = __float_as_uint(__half2float(__ushort_as_half(sc_bits)));
+        const unsigned long long s2 = (static_cast<unsigned long long>(sc) << 32) | sc;
+        if (g + 1 < G) sc_bits = __ldg(srow + g + 1);
+        const std::uint32_t db = git % C::kDB;
+        const std::uint32_t use = git / C::kDB;
+        const bool ok = tc_wait(&sm->d_full[h][db], use & 1u, abort_flag);
+        alive = __all_sync(0xffffffffu, ok);
+        if (!alive) break;
+        tc_fence_after();
+        const std::uint32_t d_addr = d_base + slot * C::kSlot;
+#pragma unroll
+        for (int c = 0; c < C::kAcc / 32; ++c) {
+          std::uint32_t d[32];
+          tmem_ld_cols<32>(d_addr + c * 32, d);
+          if (c == C::kAcc / 32 - 1) {
+            // the sums are in registers: hand the slot back before the arithmetic
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm->d_free[h][db]);
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) fma_f32x2(acc[c * 16 + i], d[2 * i], d[2 * i + 1], s2);
+        }
+        slot += C::kSub;
+        if (slot >= C::kD) slot -= C::kD;
+      }
+      if (!alive) break;
+      // ---- outputs: [activation row][weight row], a warp stores 32 consecutive rows ----
+      const int tok0 = t * NT + f * C::kAcc;
+      const int n_tok = L.M - tok0;  // may be negative: nothing to store
+      if (pair) {
+        // An even lane holds the gate and its odd neighbour the up output of one row: they
+        // exchange one of every two values, and each finishes one activation row.
+        std::uint16_t* yp = L.y + static_cast<std::size_t>(tok0 + (lane & 1)) * N + row;
+#pragma unroll
+        for (int n = 0; n < C::kAcc; n += 2) {
+          const std::uint32_t mine = pack_bf16x2(lo_f(acc[n / 2]), hi_f(acc[n / 2]));
+          const std::uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
+          const std::uint16_t gate = static_cast<std::uint16_t>((lane & 1) ? other >> 16 : mine);
+          const std::uint16_t up = static_cast<std::uint16_t>((lane & 1) ? mine >> 16 : other);
+          if (row_ok && n + (lane & 1) < n_tok) {
+            // CUDALM's rounding order: bf16 after each projection, after silu, after the product
+            yp[static_cast<std::size_t>(n) * N] =
+                float_to_bf16_bits(bf16_bits_to_float(silu_bits(gate)) * bf16_bits_to_float(up));
+          }
+        }
+      } else if (EXTRA && L.mode == kRowsResidual) {
+        std::uint16_t* yp = L.y + static_cast<std::size_t>(tok0) * N + row;
+        const std::uint16_t* rp = L.res + static_cast<std::size_t>(tok0) * N + row;
+#pragma unroll
+        for (int c = 0; c < C::kAcc; c += 16) {
+          std::uint16_t r[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            r[i] = (row_ok && c + i < n_tok) ? rp[static_cast<std::size_t>(c + i) * N] : std::uint16_t{0};
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const unsigned long long v = acc[(c + i) / 2];
+            if (row_ok && c + i < n_tok)
+              yp[static_cast<std::size_t>(c + i) * N] =
+                  add_bits(r[i], float_to_bf16_bits((i & 1) ? hi_f(v) : lo_f(v)));
+          }
+        }
+      } else {
+        std::uint16_t* yp = L.y + static_cast<std::size_t>(tok0) * N + row;
+#pragma unroll
+        for (int n = 0; n < C::kAcc; ++n) {
+          const unsigned long long v = acc[n / 2];
+          if (row_ok && n < n_tok)
+            yp[static_cast<std::size_t>(n) * N] = float_to_bf16_bits((n & 1) ? hi_f(v) : lo_f(v));
+        }
+      }
+    }
+  }
+
+  __syncthreads();
+  if (*abort_flag && tid == 0) atomicExch(p.status, CUDALM_B200_ERR_TIMEOUT);
+  tc_fence_after();
+  if (warp == 0) tmem_dealloc(tmem_d, 512);
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+template <int NT, bool EXTRA>
+int rows_launch(const RowsParams& p, cudaStream_t stream) {
+  auto kern = w4a16_rows_kernel<NT, EXTRA>;
+  constexpr int smem = rows_smem_bytes<NT>();
+  static_assert(smem <= kMaxSmemBytes, "shared memory");
+  static std::mutex mu;
+  static std::vector<int> done;
+  int dev = 0;
+  CB200_CUDA_TRY(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    bool seen = false;
+    for (int d : done) seen |= (d == dev);
+    if (!seen) {
+      CB200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      done.push_back(dev);
+    }
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.total_units < num_sms() ? p.total_units : num_sms()));
+  cfg.blockDim = dim3(kRowsThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p);
+  if (le != cudaSuccess) {
+    g_last_cuda_error = static_cast<int>(le);
+    (void)cudaGetLastError();
+    return CUDALM_B200_ERR_CUDA;
+  }
+  return check_launch();
+}
+
+template <int NT>
+int rows_launch_any(const RowsParams& p, bool extra, cudaStream_t stream) {
+  return extra ? rows_launch<NT, true>(p, stream) : rows_launch<NT, false>(p, stream);
+}
+
+}  // namespace
+
+// True when the many-row kernel takes this projection: the TMA unit needs 16-byte aligned
+// bases for the weights and activations (their row pitches are multiples of 64 bytes).
+bool rows_eligible(const cudalm_b200_linear& l) {
+  if (l.M < 1 || l.K <= 0 || (l.K % 128) != 0 || l.N < 1) return false;
+  return aligned_to(l.weight, 16) && aligned_to(l.x, 16);
+}
+
+// Up to CUDALM_B200_MAX_INLINE_LINEARS projections in one launch.  A single one may carry
+// an MLP epilogue: weight2/scales2 non-null -> y = silu(W x) * (W2 x), residual non-null ->
+// y = residual + W x.
+int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight2, const std::uint16_t* scales2,
+             const std::uint16_t* residual, cudaStream_t stream) {
+  if (count < 1 || count > CUDALM_B200_MAX_INLINE_LINEARS) return CUDALM_B200_ERR_BAD_SHAPE;
+  const bool pair = weight2 != nullptr;
+  if (pair && (!aligned_to(weight2, 16) || !scales2)) return CUDALM_B200_ERR_UNSUPPORTED;
+  for (int i = 0; i < count; ++i)
+    if (!rows_eligible(ls[i])) return CUDALM_B200_ERR_UNSUPPORTED;
+  const int tile_rows = pair ? 64 : 128;
+  // The tile that finishes first: the most loaded SM's groups times what a group costs
+  // with that many activation rows.
+  static constexpr int kTiles[3] = {256, 128, 64};
+  static constexpr int kCycles[3] = {1150, 650, 420};
+  int nt = 0;
+  long long best = 0;
+  for (int k = 0; k < 3; ++k) {
+    long long groups = 0, units = 0, longest = 0;
+    for (int i = 0; i < count; ++i) {
+      const long long n = static_cast<long long>((ls[i].N + tile_rows - 1) / tile_rows) *
+                          ((ls[i].M + kTiles[k] - 1) / kTiles[k]);
+      units += n;
+      groups += n * (ls[i].K >> 7);
+      if ((ls[i].K >> 7) > longest) longest = ls[i].K >> 7;
+    }
+    if (units > 0x3fffffff || groups > 0x3fffffff) return CUDALM_B200_ERR_TOO_LARGE;
+    const long long rounds = (units + num_sms() - 1) / num_sms();
+    long long load = count == 1 ? rounds * longest : (groups + num_sms() - 1) / num_sms() + longest / 2;
+    if (load < longest) load = longest;
+    if (nt == 0 || load * kCycles[k] < best) {
+      best = load * kCycles[k];
+      nt = kTiles[k];
+    }
+  }
+  RowsParams p;
+  std::memset(&p, 0, sizeof(p));
+  int units = 0, cost = 0;
+  for (int i = 0; i < count; ++i) {
+    const cudalm_b200_linear& l = ls[i];
+    RowsDesc& d = p.d[i];
+    if (int rc = tc_encode(l.weight, l.K / 8, l.N, 32, tile_rows, 0, &d.tmap)) return rc;
+    if (pair)
+      if (int rc = tc_encode(weight2, l.K / 8, l.N, 32, tile_rows, 0, &d.tmap2)) return rc;
+    if (int rc = tc_encode(l.x, l.K, l.M, 64, nt, 1, &d.xmap)) return rc;
+    d.S = l.scales;
+    d.S2 = scales2;
+    d.res = residual;
+    d.y = l.y;
+    d.N = l.N;
+    d.K = l.K;
+    d.M = l.M;
+    d.mode = pair ? kRowsPair : (residual ? kRowsResidual : kRowsPlain);
+    d.tok_tiles = (l.M + nt - 1) / nt;
+    d.unit_begin = units;
+    d.cost_begin = cost;
+    const int n = (l.N + tile_rows - 1) / tile_rows * d.tok_tiles;
+    units += n;
+    cost += n * (l.K >> 7);
+    d.unit_end = units;
+  }
+  p.n_desc = count;
+  p.total_units = units;
+  p.total_cost = cost;
+  p.status = device_status_word();
+  if (!p.status) return CUDALM_B200_ERR_CUDA;
+  const bool extra = pair || residual;
+  if (nt == 256) return rows_launch_any<256>(p, extra, stream);
+  if (nt == 128) return rows_launch_any<128>(p, extra, stream);
+  return rows_launch_any<64>(p, extra, stream);
+}
+
+}  // namespace cb200

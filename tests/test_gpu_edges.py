@@ -3,7 +3,7 @@
 import numpy as np
 import pytest
 
-from helpers import BASE_SEED, check_close, from_dev, make_x, raw_weights, to_dev
+from helpers import BASE_SEED, _ordinal, check_close, from_dev, make_x, raw_weights, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -82,3 +82,58 @@ def test_quantizer_group_counts(eng, orc, N, K):
     """Group counts around a warp's sixteen and around a whole grid of them."""
     rng = np.random.default_rng(BASE_SEED + N)
     _quantize_equal(eng, orc, orc.f32_to_bf16_bits((rng.standard_normal((N, K)) * 0.02).astype(np.float32)))
+
+
+# the many-row kernel: activation tiles of 64 (few units), 128 and 256 rows; tile remainders of
+# either side; one group, an odd number of groups and more groups than any ring holds
+ROWS_SHAPES = [(1, 128, 65), (63, 128, 129), (64, 256, 127), (127, 384, 128), (129, 2944, 66),
+               (513, 4608, 96), (1023, 256, 2048), (1024, 384, 2047), (4100, 128, 2085), (4224, 640, 1793),
+               (19000, 128, 70)]
+
+
+@pytest.mark.parametrize("N,K,M", ROWS_SHAPES)
+def test_many_rows(eng, orc, N, K, M):
+    """Plain, residual (also in place) and gate/up forms above 64 rows against the oracle,
+    and twice for equal bits; outputs off 16 bytes and off the matrix stay untouched."""
+    import torch
+    W, S = raw_weights(N, K, BASE_SEED + N)
+    x = make_x(orc, (M, K), BASE_SEED + M, "outlier")
+    want = orc.batch_gemv_bf16(W, S, x, threads=8)
+    Wd, Sd, xd = to_dev(W), to_dev(S, torch.float16), to_dev(x, torch.bfloat16)
+    buf = torch.full((M * N + 3,), 7.0, device="cuda", dtype=torch.bfloat16)
+    y = buf[1:1 + M * N].view(M, N)
+    got = from_dev(eng.batch_int4_gemv_bf16(Wd, Sd, xd, y))
+    check_close(orc, got, want, f"{N}x{K} M={M}")
+    assert buf[0] == 7.0 and bool((buf[1 + M * N:] == 7.0).all())
+    assert np.array_equal(got, from_dev(eng.batch_int4_gemv_bf16(Wd, Sd, xd)))
+
+    lin = eng.W4A16Linear(Wd, Sd)
+    res = make_x(orc, (M, N), BASE_SEED + 1)
+    h = to_dev(res, torch.bfloat16)
+    want_res = orc.add_bf16(res.ravel(), got.ravel()).reshape(M, N)
+    assert np.array_equal(from_dev(eng.linear_residual_bf16(lin, xd, h)), want_res)
+    assert np.array_equal(from_dev(eng.linear_residual_bf16(lin, xd, h, y=h)), want_res)
+
+    W2, S2 = raw_weights(N, K, BASE_SEED + N + 1)
+    up = eng.W4A16Linear(to_dev(W2), to_dev(S2, torch.float16))
+    g_y, u_y = eng.gate_up_bf16(lin, up, xd)
+    assert np.array_equal(from_dev(g_y), got)
+    fused = from_dev(eng.gate_up_silu_bf16(lin, up, xd))
+    two = orc.silu_mul_bf16(from_dev(g_y).ravel(), from_dev(u_y).ravel()).reshape(M, N)
+    off = _ordinal(fused) - _ordinal(two)
+    assert np.abs(off).max() <= 1 and np.count_nonzero(off) <= max(2, 2e-3 * off.size)
+
+
+def test_many_rows_in_one_call_with_few(eng, orc):
+    """linear_multi over projections of different shapes and row counts, some below 65 rows."""
+    import torch
+    items, want = [], []
+    for i, (N, K, M) in enumerate([(300, 384, 200), (16, 1024, 3), (1000, 128, 65), (129, 256, 500)]):
+        W, S = raw_weights(N, K, BASE_SEED + i)
+        x = make_x(orc, (M, K), BASE_SEED + i)
+        want.append(orc.batch_gemv_bf16(W, S, x, threads=8))
+        items.append((eng.W4A16Linear(to_dev(W), to_dev(S, torch.float16)), to_dev(x, torch.bfloat16),
+                      torch.empty((M, N), device="cuda", dtype=torch.bfloat16)))
+    eng.linear_multi(items)
+    for (_, _, y), w in zip(items, want):
+        check_close(orc, from_dev(y), w)
