@@ -42,7 +42,7 @@ namespace cb200 {
 constexpr int kDirectWarps = 8;
 constexpr int kDirectThreads = kDirectWarps * 32;
 constexpr int kDirectBatch = 4;     // groups whose weights a lane holds in registers at once
-constexpr int kDirectMaxRows = 8;   // activation rows (the 8 columns of the MMA)
+constexpr int kDirectMaxRows = 16;  // activation rows: one or two MMA column tiles of 8
 
 enum : int { kDirectPlain = 0, kDirectPair = 1, kDirectResidual = 2 };
 
@@ -98,33 +98,50 @@ __device__ __forceinline__ void dequant_pairs(std::uint32_t w, std::uint32_t (&o
     out[i] = sub_bf16x2(lop3_and_xor(w >> (4 * i), 0x000F000Fu, kMagic), kMagic);
 }
 
-// One quantisation group of rows (r8, r8 + 8): sum[0..3] = the group's four sums
-// of the lane's fragment (rows r8 / r8 + 8, activation rows 2t / 2t + 1).
-__device__ __forceinline__ void direct_group(const uint4& qa, const uint4& qb, const uint4 (&X)[4],
-                                             float (&sum)[4]) {
+// One quantisation group of rows (r8, r8 + 8): sum[n][0..3] = the group's four sums of the
+// lane's fragment (rows r8 / r8 + 8, activation rows 8 n + 2t / 2t + 1).  `xr[n]` points to
+// the lane's 32 activations of row 8 n + r8; rows past M (x_real[n] false) count as zeros.
+template <int NCOL>
+__device__ __forceinline__ void direct_group(const uint4& qa, const uint4& qb,
+                                             const std::uint16_t* const (&xr)[NCOL], const bool (&x_real)[NCOL],
+                                             int x_off, float (&sum)[NCOL][4]) {
   const std::uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w};
   const std::uint32_t wb[4] = {qb.x, qb.y, qb.z, qb.w};
-  float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+  uint4 X[NCOL][4];
+#pragma unroll
+  for (int n = 0; n < NCOL; ++n)
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+      X[n][w] = x_real[n] ? ldg_activations(xr[n] + x_off + w * 8) : make_uint4(0u, 0u, 0u, 0u);
+  float c0[NCOL][4] = {}, c1[NCOL][4] = {};
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
     std::uint32_t A[4], B[4];
     dequant_pairs(wa[w], A);
     dequant_pairs(wb[w], B);
-    // activations k = 8 w + {0..7} of this lane's 32: pairs (i, i + 4) to match the weights
-    const std::uint32_t b00 = __byte_perm(X[w].x, X[w].z, 0x5410);  // {x0, x4}
-    const std::uint32_t b01 = __byte_perm(X[w].x, X[w].z, 0x7632);  // {x1, x5}
-    const std::uint32_t b10 = __byte_perm(X[w].y, X[w].w, 0x5410);  // {x2, x6}
-    const std::uint32_t b11 = __byte_perm(X[w].y, X[w].w, 0x7632);  // {x3, x7}
-    mma_m16n8k16_bf16(c0, A[0], B[0], A[1], B[1], b00, b01);
-    mma_m16n8k16_bf16(c1, A[2], B[2], A[3], B[3], b10, b11);
+#pragma unroll
+    for (int n = 0; n < NCOL; ++n) {
+      // activations k = 8 w + {0..7} of this lane's 32: pairs (i, i + 4) to match the weights
+      const uint4& v = X[n][w];
+      const std::uint32_t b00 = __byte_perm(v.x, v.z, 0x5410);  // {x0, x4}
+      const std::uint32_t b01 = __byte_perm(v.x, v.z, 0x7632);  // {x1, x5}
+      const std::uint32_t b10 = __byte_perm(v.y, v.w, 0x5410);  // {x2, x6}
+      const std::uint32_t b11 = __byte_perm(v.y, v.w, 0x7632);  // {x3, x7}
+      mma_m16n8k16_bf16(c0[n], A[0], B[0], A[1], B[1], b00, b01);
+      mma_m16n8k16_bf16(c1[n], A[2], B[2], A[3], B[3], b10, b11);
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) sum[i] = c0[i] + c1[i];
+  for (int n = 0; n < NCOL; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[n][i] = c0[n][i] + c1[n][i];
 }
 
-__global__ void __launch_bounds__(kDirectThreads, 3)
+// NCOL: tiles of 8 activation rows.
+template <int NCOL>
+__global__ void __launch_bounds__(kDirectThreads, NCOL == 1 ? 3 : 2)
 w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
-  __shared__ float4 red[2][kDirectWarps][32];
+  __shared__ float4 red[2][NCOL][kDirectWarps][32];
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
@@ -145,8 +162,8 @@ w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
   const int row0 = (tile0 + tile_in_cta) * 16;
   const bool active = tile_in_cta < d.tiles_per_cta && row0 < N;
 
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};   // the projection, or the gate matrix of a pair
-  float acc2[4] = {0.f, 0.f, 0.f, 0.f};  // the up matrix of a pair
+  float acc[NCOL][4] = {};   // the projection, or the gate matrix of a pair
+  float acc2[NCOL][4] = {};  // the up matrix of a pair
   bool waited = false;
   if (active) {
     const int r8 = lane >> 2, t = lane & 3;
@@ -156,8 +173,13 @@ w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
     const std::size_t wb_off = static_cast<std::size_t>(rb) * (K >> 1) + t * 16;
     const std::size_t sa_off = static_cast<std::size_t>(ra) * G;
     const std::size_t sb_off = static_cast<std::size_t>(rb) * G;
-    const bool x_real = r8 < M;  // MMA columns past M are fed zeros
-    const std::uint16_t* xr = d.x + static_cast<std::size_t>(x_real ? r8 : 0) * K + t * 32;
+    bool x_real[NCOL];  // MMA columns past M are fed zeros
+    const std::uint16_t* xr[NCOL];
+#pragma unroll
+    for (int n = 0; n < NCOL; ++n) {
+      x_real[n] = 8 * n + r8 < M;
+      xr[n] = d.x + static_cast<std::size_t>(x_real[n] ? 8 * n + r8 : 0) * K + t * 32;
+    }
     const int gbeg = split * d.gps;
     const int gend = min(G, gbeg + d.gps);
     // A lane holds kDirectBatch (group, matrix) slots at a time: four groups of the one
@@ -188,24 +210,17 @@ w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
         const bool second = pair && j >= kDirectBatch / 2;
         const int g = g0 + (pair ? (j & (kDirectBatch / 2 - 1)) : j);
         if (g < gend) {
-          uint4 X[4];
-#pragma unroll
-          for (int w = 0; w < 4; ++w)
-            X[w] = x_real ? ldg_activations(xr + g * 128 + w * 8) : make_uint4(0u, 0u, 0u, 0u);
-          float sum[4];
-          direct_group(qa[j], qb[j], X, sum);
+          float sum[NCOL][4];
+          direct_group<NCOL>(qa[j], qb[j], xr, x_real, g * 128, sum);
           const float s_lo = __half2float(__ushort_as_half(sca[j]));
           const float s_hi = __half2float(__ushort_as_half(scb[j]));
-          if (second) {
-            acc2[0] = fmaf(s_lo, sum[0], acc2[0]);
-            acc2[1] = fmaf(s_lo, sum[1], acc2[1]);
-            acc2[2] = fmaf(s_hi, sum[2], acc2[2]);
-            acc2[3] = fmaf(s_hi, sum[3], acc2[3]);
-          } else {
-            acc[0] = fmaf(s_lo, sum[0], acc[0]);
-            acc[1] = fmaf(s_lo, sum[1], acc[1]);
-            acc[2] = fmaf(s_hi, sum[2], acc[2]);
-            acc[3] = fmaf(s_hi, sum[3], acc[3]);
+#pragma unroll
+          for (int n = 0; n < NCOL; ++n) {
+            float (&a)[4] = second ? acc2[n] : acc[n];
+            a[0] = fmaf(s_lo, sum[n][0], a[0]);
+            a[1] = fmaf(s_lo, sum[n][1], a[1]);
+            a[2] = fmaf(s_hi, sum[n][2], a[2]);
+            a[3] = fmaf(s_hi, sum[n][3], a[3]);
           }
         }
       }
@@ -213,27 +228,30 @@ w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
   }
   if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  red[0][warp][lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-  if (pair) red[1][warp][lane] = make_float4(acc2[0], acc2[1], acc2[2], acc2[3]);
+#pragma unroll
+  for (int n = 0; n < NCOL; ++n) {
+    red[0][n][warp][lane] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+    if (pair) red[1][n][warp][lane] = make_float4(acc2[n][0], acc2[n][1], acc2[n][2], acc2[n][3]);
+  }
   __syncthreads();
 
-  // Outputs of the CTA's m-tiles: (row r, activation row c) of a tile sits in lane
+  // Outputs of the CTA's m-tiles: (row r, activation row 8 n + c) of a tile sits in lane
   // (r % 8) * 4 + c / 2, element (r / 8) * 2 + c % 2 of each of the tile's warps.
-  const int n_out = d.tiles_per_cta * 128;
+  const int n_out = d.tiles_per_cta * 128 * NCOL;
   for (int idx = tid; idx < n_out; idx += kDirectThreads) {
-    const int tile = idx >> 7, c = (idx >> 4) & 7, r = idx & 15;
-    const int row = (tile0 + tile) * 16 + r;
-    if (c >= M || row >= N) continue;
+    const int r = idx & 15, c = (idx >> 4) & 7, n = (idx >> 7) % NCOL, tile = (idx >> 7) / NCOL;
+    const int row = (tile0 + tile) * 16 + r, col = 8 * n + c;
+    if (col >= M || row >= N) continue;
     const int src_lane = (r & 7) * 4 + (c >> 1);
     const int elem = (r >> 3) * 2 + (c & 1);
     const int w0 = tile * nsplit;
     float v = 0.f;
-    for (int s = 0; s < nsplit; ++s) v += reinterpret_cast<const float*>(&red[0][w0 + s][src_lane])[elem];
+    for (int s = 0; s < nsplit; ++s) v += reinterpret_cast<const float*>(&red[0][n][w0 + s][src_lane])[elem];
     std::uint16_t o = float_to_bf16_bits(v);
-    const std::size_t at = static_cast<std::size_t>(c) * N + row;
+    const std::size_t at = static_cast<std::size_t>(col) * N + row;
     if (pair) {
       float u = 0.f;
-      for (int s = 0; s < nsplit; ++s) u += reinterpret_cast<const float*>(&red[1][w0 + s][src_lane])[elem];
+      for (int s = 0; s < nsplit; ++s) u += reinterpret_cast<const float*>(&red[1][n][w0 + s][src_lane])[elem];
       // CUDALM's rounding order (src/kernels/qwen35_kernels.cu:459-476)
       o = silu_mul_bits(bf16_bits_to_float(o), float_to_bf16_bits(u));
     } else if (mode == kDirectResidual) {
@@ -298,6 +316,8 @@ int run_direct(const cudalm_b200_linear* ls, int count, const std::uint8_t* cons
     if (ctas > 0x7fffffff) return CUDALM_B200_ERR_TOO_LARGE;
   }
   p.n_desc = count;
+  int mmax = 0;
+  for (int i = 0; i < count; ++i) mmax = ls[i].M > mmax ? ls[i].M : mmax;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas));
   cfg.blockDim = dim3(kDirectThreads);
@@ -308,7 +328,7 @@ int run_direct(const cudalm_b200_linear* ls, int count, const std::uint8_t* cons
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, w4a16_direct_kernel, p);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, mmax <= 8 ? w4a16_direct_kernel<1> : w4a16_direct_kernel<2>, p);
   if (le != cudaSuccess) {
     g_last_cuda_error = static_cast<int>(le);
     (void)cudaGetLastError();
@@ -319,7 +339,7 @@ int run_direct(const cudalm_b200_linear* ls, int count, const std::uint8_t* cons
 
 int direct_kernel_regs() {
   cudaFuncAttributes attr;
-  if (cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(&w4a16_direct_kernel)) != cudaSuccess) {
+  if (cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(&w4a16_direct_kernel<1>)) != cudaSuccess) {
     (void)cudaGetLastError();
     return -1;
   }

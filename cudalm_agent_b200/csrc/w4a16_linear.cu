@@ -378,12 +378,19 @@ int run_fallback(const cudalm_b200_linear& l, cudaStream_t stream) {
   return check_launch();
 }
 
+// True when the lean kernel answers a single call: up to g_direct_max_bytes of weights, and
+// any number of bytes where K is beyond the streaming kernel's shared memory (K > 4096: the
+// other choice is the one-warp-per-row kernel; 8192 x 8192, one row: 65.6 -> 16.4 us).
+bool direct_takes(const cudalm_b200_linear& l, const std::uint8_t* weight2) {
+  if (!direct_eligible(l, weight2)) return false;
+  const long long limit = g_direct_max_bytes.load(std::memory_order_relaxed);
+  return direct_weight_bytes(l, weight2 != nullptr) <= limit || (limit > 0 && l.K > kMaxStreamK);
+}
+
 // One projection with any M: passes of as many rows as fit in shared memory.
 int run_single(cudalm_b200_linear l, cudaStream_t stream) {
   if (int rc = validate(l)) return rc;
-  if (direct_eligible(l, nullptr) &&
-      direct_weight_bytes(l, false) <= g_direct_max_bytes.load(std::memory_order_relaxed))
-    return run_direct(&l, 1, nullptr, nullptr, nullptr, stream);
+  if (direct_takes(l, nullptr)) return run_direct(&l, 1, nullptr, nullptr, nullptr, stream);
   if (l.M >= g_tc_min_rows.load(std::memory_order_relaxed)) {
     // the tensor-memory kernels: one for up to 64 rows, one for any number above
     if (l.M <= kTcMaxRows && tc_eligible(l)) return run_tc(&l, 1, stream);
@@ -416,8 +423,7 @@ int run_extra(cudalm_b200_linear l, const LinearExtra& ex, cudaStream_t stream) 
   if (int rc = validate(l)) return rc;
   const bool pair = ex.weight2 != nullptr;
   if (pair && !ex.scales2) return CUDALM_B200_ERR_NULL;
-  if (direct_eligible(l, ex.weight2) &&
-      direct_weight_bytes(l, pair) <= g_direct_max_bytes.load(std::memory_order_relaxed)) {
+  if (direct_takes(l, ex.weight2)) {
     const std::uint8_t* w2[1] = {ex.weight2};
     const std::uint16_t* s2[1] = {ex.scales2};
     const std::uint16_t* rs[1] = {ex.residual};

@@ -137,3 +137,33 @@ def test_many_rows_in_one_call_with_few(eng, orc):
     eng.linear_multi(items)
     for (_, _, y), w in zip(items, want):
         check_close(orc, from_dev(y), w)
+
+
+@pytest.mark.parametrize("N,K,M", [(1, 128, 9), (17, 384, 16), (40, 1152, 10), (5003, 2944, 13), (1000, 1024, 15),
+                                   (33, 4224, 1), (100, 8192, 8), (257, 8320, 16), (15, 16384, 9), (700, 4096, 12)])
+def test_lean_kernel_up_to_sixteen_rows_and_any_k(eng, orc, N, K, M):
+    """One and two column tiles, K splits of equal and unequal length, K beyond the
+    streaming kernel's limit: plain, residual and gate/up forms against the oracle."""
+    import torch
+    W, S = raw_weights(N, K, BASE_SEED + N)
+    W2, S2 = raw_weights(N, K, BASE_SEED + N + 1)
+    x = make_x(orc, (M, K), BASE_SEED + M, "outlier")
+    res = make_x(orc, (M, N), BASE_SEED + 1)
+    want = orc.batch_gemv_bf16(W, S, x, threads=8)
+    lin, up = (eng.W4A16Linear(to_dev(w), to_dev(s, torch.float16)) for w, s in ((W, S), (W2, S2)))
+    xd = to_dev(x, torch.bfloat16)
+    prev = eng.set_direct_path_max_bytes(1 << 40)
+    try:
+        got = from_dev(eng.batch_int4_gemv_bf16(lin.weight, lin.scale, xd))
+        other = from_dev(eng.batch_int4_gemv_bf16(up.weight, up.scale, xd))
+        added = from_dev(eng.linear_residual_bf16(lin, xd, to_dev(res, torch.bfloat16)))
+        fused = from_dev(eng.gate_up_silu_bf16(lin, up, xd))
+        for m in {0, M // 2, M - 1}:  # a row's bits do not depend on its batch
+            assert np.array_equal(from_dev(eng.int4_gemv_bf16(lin.weight, lin.scale, xd[m].contiguous())), got[m])
+    finally:
+        eng.set_direct_path_max_bytes(prev)
+    check_close(orc, got, want, f"{N}x{K} M={M}")
+    assert np.array_equal(added, orc.add_bf16(res.ravel(), got.ravel()).reshape(M, N))
+    two = orc.silu_mul_bf16(got.ravel(), other.ravel()).reshape(M, N)
+    off = _ordinal(fused) - _ordinal(two)
+    assert np.abs(off).max() <= 1 and np.count_nonzero(off) <= max(2, 2e-3 * off.size)
