@@ -113,6 +113,7 @@ SIGNATURES = {
 }
 
 _lib: Optional[ctypes.CDLL] = None
+_native = None  # the compiled binding of the calls a decode loop issues step by step
 
 
 def library_path() -> str:
@@ -122,7 +123,7 @@ def library_path() -> str:
 
 def load_library() -> ctypes.CDLL:
     """Loads ``libcudalm_b200.so`` (it must have been built; see ``build.py``)."""
-    global _lib
+    global _lib, _native
     if _lib is None:
         path = library_path()
         if not os.path.exists(path):
@@ -133,8 +134,30 @@ def load_library() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.restype = res
             fn.argtypes = args
+        _native = _load_binding(lib)
         _lib = lib
     return _lib
+
+
+def _load_binding(lib: ctypes.CDLL):
+    try:
+        from . import _native as binding
+    except ImportError as e:
+        raise CudalmB200Error("load_library", ERR_UNSUPPORTED,
+                              f"{_build.BINDING_PATH} does not load ({e}): run python -m "
+                              "cudalm_agent_b200.build")
+    binding.bind(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in (
+        "cudalm_b200_int4_gemv_bf16", "cudalm_b200_batch_int4_gemv_bf16", "cudalm_b200_linear_multi",
+        "cudalm_b200_gate_up_silu_bf16", "cudalm_b200_linear_residual_bf16")))
+    return binding
+
+
+def _bound():
+    """The binding.  Its functions return a status, or -1 for a call they leave to the
+    checks below them (see binding.cpp)."""
+    if _native is None:
+        load_library()
+    return _native
 
 
 def _check(fn: str, status: int) -> None:
@@ -241,6 +264,12 @@ def int4_gemv_bf16(weight: torch.Tensor, scales: torch.Tensor, x: torch.Tensor,
                    K: Optional[int] = None) -> torch.Tensor:
     """``y[n] = sum_k q[n,k] * scale[n,k/128] * x[k]`` (CUDALM
     include/cudalm/kernels/int4_gemv_bf16.h:46-48).  x bf16 ``[K]`` -> y bf16 ``[N]``."""
+    if y is not None and N is None and K is None:
+        st = _bound().gemv(weight, scales, x, y)
+        if st >= 0:
+            if st:
+                _check("int4_gemv_bf16", st)
+            return y
     _need(weight, torch.uint8, "weight")
     _need(scales, torch.float16, "scales")
     _need(x, torch.bfloat16, "x")
@@ -262,6 +291,12 @@ def batch_int4_gemv_bf16(weight: torch.Tensor, scales: torch.Tensor, x: torch.Te
                          K: Optional[int] = None, B: Optional[int] = None) -> torch.Tensor:
     """B rows against the same weights (CUDALM include/cudalm/kernels/batch_decode.h:61-63):
     x bf16 ``[B, K]`` -> y bf16 ``[B, N]``."""
+    if y is not None and N is None and K is None and B is None:
+        st = _bound().batch(weight, scales, x, y)
+        if st >= 0:
+            if st:
+                _check("batch_int4_gemv_bf16", st)
+            return y
     _need(weight, torch.uint8, "weight")
     _need(scales, torch.float16, "scales")
     _need(x, torch.bfloat16, "x")
@@ -292,6 +327,11 @@ def _fill(desc: _LinearStruct, lin: W4A16Linear, x: torch.Tensor, y: torch.Tenso
 
 def linear_multi(items: Sequence[Tuple[W4A16Linear, torch.Tensor, torch.Tensor]]) -> None:
     """Up to four independent projections ``(linear, x, y)`` in one launch."""
+    st = _bound().multi(items)
+    if st >= 0:
+        if st:
+            _check("linear_multi", st)
+        return
     arr = (_LinearStruct * len(items))()
     for d, (lin, x, y) in zip(arr, items):
         _fill(d, lin, x, y)
@@ -343,6 +383,12 @@ def gate_up_silu_bf16(gate: W4A16Linear, up: W4A16Linear, x: torch.Tensor,
                       out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """silu(gate(x)) * up(x) in one launch, rounded as CUDALM rounds it
     (src/kernels/qwen35_kernels.cu:459-476 after the two projections)."""
+    if out is not None:
+        st = _bound().gate_up_silu(gate, up, x, out)
+        if st >= 0:
+            if st:
+                _check("gate_up_silu_bf16", st)
+            return out
     _need(x, torch.bfloat16, "x")
     if gate.N != up.N or gate.K != up.K:
         raise ValueError("gate and up must have the same shape")
@@ -361,6 +407,12 @@ def linear_residual_bf16(lin: W4A16Linear, x: torch.Tensor, residual: torch.Tens
                          y: Optional[torch.Tensor] = None) -> torch.Tensor:
     """residual + lin(x), rounded as CUDALM rounds it (projection to bf16, then
     src/kernels/qwen35_kernels.cu:442-456)."""
+    if y is not None:
+        st = _bound().linear_residual(lin, x, residual, y)
+        if st >= 0:
+            if st:
+                _check("linear_residual_bf16", st)
+            return y
     _need(x, torch.bfloat16, "x")
     _need(residual, torch.bfloat16, "residual")
     M = 1 if x.dim() == 1 else int(x.shape[0])

@@ -2,9 +2,10 @@
 
     python -m cudalm_agent_b200.build
 
-produces ``cudalm_agent_b200/lib/libcudalm_b200.so``.  The library is
-self-contained (static CUDA runtime) and exports only the C ABI declared in
-``include/cudalm_b200.h``.
+produces ``cudalm_agent_b200/lib/libcudalm_b200.so``, which is self-contained (static
+CUDA runtime) and exports only the C ABI declared in ``include/cudalm_b200.h``, and
+``cudalm_agent_b200/_native.so``, the Python binding of its most frequent calls, which is
+built against the installed torch.
 """
 from __future__ import annotations
 
@@ -16,6 +17,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libcudalm_b200.so")
+BINDING_SRC = os.path.join(CSRC, "binding.cpp")
+BINDING_PATH = os.path.join(PKG, "_native.so")
 
 SOURCES = ["runtime.cu", "w4a16_linear.cu", "w4a16_tc.cu", "w4a16_rows.cu", "w4a16_direct.cu", "quantize.cu", "lm_head.cu", "sample.cu",
            "weights_v2.cu"]
@@ -34,12 +37,27 @@ def _nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(BINDING_PATH):
         return True
-    t = os.path.getmtime(LIB_PATH)
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(BINDING_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(os.path.dirname(PKG), "include", "cudalm_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _compile_binding():
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include",
+           f"-I{sysconfig.get_paths()['include']}", "-o", BINDING_PATH, BINDING_SRC,
+           f"-L{root}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    return BINDING_PATH, res.returncode, res.stdout + res.stderr
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
@@ -70,8 +88,13 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         res = subprocess.run(cmd, capture_output=True, text=True)
         return obj, res.returncode, res.stdout + res.stderr
 
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
+        binding = ex.submit(_compile_binding)
         results = list(ex.map(compile_one, srcs))
+        _, rc, out = binding.result()
+    if rc != 0:
+        sys.stderr.write(out)
+        raise RuntimeError("g++ failed building _native.so")
     for _, rc, out in results:
         if verbose or rc != 0:
             sys.stderr.write(out)

@@ -167,3 +167,57 @@ def test_lean_kernel_up_to_sixteen_rows_and_any_k(eng, orc, N, K, M):
     two = orc.silu_mul_bf16(got.ravel(), other.ravel()).reshape(M, N)
     off = _ordinal(fused) - _ordinal(two)
     assert np.abs(off).max() <= 1 and np.count_nonzero(off) <= max(2, 2e-3 * off.size)
+
+
+def test_bound_calls_take_and_refuse_what_the_checks_do(eng):
+    """The compiled binding answers exactly the calls the Python checks would pass on, and
+    leaves the rest to them: the same bits through either, the same errors as without it."""
+    import torch
+    from cudalm_agent_b200 import api
+    W, S = raw_weights(64, 256, BASE_SEED)
+    W2, S2 = raw_weights(64, 256, BASE_SEED + 1)
+    l1, l2 = (eng.W4A16Linear(to_dev(w), to_dev(s, torch.float16)) for w, s in ((W, S), (W2, S2)))
+    x = torch.randn(5, 256, device="cuda").bfloat16()
+    res, y = torch.randn(5, 64, device="cuda").bfloat16(), torch.empty(5, 64, device="cuda", dtype=torch.bfloat16)
+    calls = [
+        lambda x, y: eng.int4_gemv_bf16(l1.weight, l1.scale, x[0], y[0]),
+        lambda x, y: eng.batch_int4_gemv_bf16(l1.weight, l1.scale, x, y),
+        lambda x, y: eng.linear_multi([(l1, x, y)]),
+        lambda x, y: eng.gate_up_silu_bf16(l1, l2, x, y),
+        lambda x, y: eng.linear_residual_bf16(l1, x, res, y),
+    ]
+    native = api._native
+
+    class Off:
+        def __getattr__(self, name):
+            return lambda *a: -1
+
+    for i, call in enumerate(calls):
+        out = []
+        for binding in (native, Off()):
+            api._native = binding
+            try:
+                y.zero_()
+                call(x, y)
+                out.append(from_dev(y).copy())
+                for bad_x, bad_y in ((x.float(), y), (x.cpu(), y), (x, y.float()), (x.t().contiguous().t(), y)):
+                    if i > 2 and bad_y is not y:
+                        continue  # these two take the output as it is
+                    with pytest.raises(ValueError):
+                        call(bad_x, bad_y)
+                if i in (0, 1):
+                    with pytest.raises(ValueError):
+                        call(x[:, :128].contiguous(), y)
+            finally:
+                api._native = native
+        assert np.array_equal(out[0], out[1]), i
+    assert native.batch(l1.weight, l1.scale, x, y) == 0
+    assert native.batch(l1.weight, l1.scale, x.t().contiguous().t(), y) == -1
+    assert native.batch(l1.weight, l1.scale, x, y[:, :32]) == -1
+    assert native.linear_residual(l1, x, res[:, :63], y) == -1
+    assert native.gate_up_silu(l1, None, x, y) == -1
+    assert native.multi([(l1, x, y)] * 5) == -1 and native.multi([]) == -1
+    seen = []  # a wrapped tensor is not taken
+    torch.func.vmap(lambda v: seen.append(native.gemv(l1.weight, l1.scale, v, y[0])) or v)(x)
+    assert seen == [-1]
+    torch.cuda.synchronize()
