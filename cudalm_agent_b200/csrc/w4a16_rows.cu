@@ -41,14 +41,17 @@ struct alignas(64) RowsDesc {
   CUtensorMap tmap;   // weights as uint32 [N][K/8], box 128 rows (a pair: 64) x 32 words
   CUtensorMap tmap2;  // kRowsPair: the second (up) matrix
   CUtensorMap xmap;   // activations as bf16 [M][K], box NT rows x 64 values
+  CUtensorMap ymap;   // outputs as bf16 [M][N], box 32 rows x 128 values (a pair: 64)
+  CUtensorMap rmap;   // kRowsResidual: the residual, box as ymap
   const std::uint16_t* S;
   const std::uint16_t* S2;   // kRowsPair: scales of the second matrix
   const std::uint16_t* res;  // kRowsResidual: residual [M][N]; may be y
   std::uint16_t* y;
   int N, K, M;
   int mode;
-  int tok_tiles;   // unit = weight tile * tok_tiles + activation tile
-  int unit_begin;  // first unit of this projection in the launch
+  int direct_store;  // outputs (or the residual) are not what the TMA unit takes
+  int tok_tiles;     // unit = weight tile * tok_tiles + activation tile
+  int unit_begin;    // first unit of this projection in the launch
   int unit_end;
   int cost_begin;  // groups before this projection
 };
@@ -70,28 +73,33 @@ struct RowsCfg {
   static constexpr int kSlot = NT / kSub;                // columns of an accumulator slot
   static constexpr int kAcc = NT / 2;                    // running sums per fold thread
   static constexpr int kD = NT == 256 ? 3 : (NT == 128 ? 2 : 4);  // accumulator slots
-  // Barrier pairs per issuer.  NT = 256: the three slots go round over both issuers, so one
-  // of them can hold all three; four pairs keep it from lapping a barrier.
+  // Barriers for a freed slot.  NT = 256: the three slots go round over both halves, so one
+  // half can hold all three; four barriers keep it from lapping one.
   static constexpr int kDB = NT == 256 ? 4 : kD;
   static constexpr int kA = NT == 256 ? 2 : 4;           // A buffers of 64 columns
-  static constexpr int kW = NT == 256 ? 2 : (NT == 128 ? 4 : 6);  // weight stages, 16 KB
-  static constexpr int kB = NT == 256 ? 3 : (NT == 128 ? 4 : 6);  // activation stages
+  static constexpr int kW = NT == 256 ? 2 : (NT == 128 ? 4 : 6);   // weight stages (two groups, 16 KB)
+  static constexpr int kB = NT == 256 ? 5 : (NT == 128 ? 8 : 12);  // activation stages (half a group)
+  // Barriers for a finished group: more than any ring that waits for them reaches back.
+  static constexpr int kR = NT == 256 ? 4 : 8;
   static constexpr int kBoxBytes = NT * 128;             // NT rows x 64 values
-  static constexpr int kBBytes = 2 * kBoxBytes;
   static constexpr int kRegFold = NT == 256 ? 176 : 136;
   static constexpr int kRegDequant = NT == 256 ? 48 : 72;
   static constexpr int kRegOther = NT == 256 ? 32 : 64;
   static_assert(kD * kSlot + kA * 64 <= 512, "tensor memory");
+  static_assert(kW % 2 == 0 && kA <= kR && kB / 2 < kR, "rings");
 };
 constexpr int kRowsWBytes = kTcRowsPerTile * 128;
 constexpr int kRowsHeaderBytes = 1024;
+constexpr int kRowsChunk = 32;                                       // activation rows per output box
+constexpr int kRowsOutBytes = kRowsChunk * kTcRowsPerTile * 2;       // two of them per fold set
 template <int NT>
 constexpr int rows_smem_bytes() {
-  return 1024 + kRowsHeaderBytes + RowsCfg<NT>::kW * kRowsWBytes + RowsCfg<NT>::kB * RowsCfg<NT>::kBBytes;
+  return 1024 + kRowsHeaderBytes + RowsCfg<NT>::kW * kRowsWBytes + RowsCfg<NT>::kB * RowsCfg<NT>::kBoxBytes +
+         4 * kRowsOutBytes;
 }
 
-// Warp roles: 0..3 and 4..7 dequantise even / odd groups, 8..11 and 12..15 fold (each half
-// of the activation rows), 16 copies weights, 18 activations, 17 and 19 issue MMAs.
+// Warp roles: 0..3 and 4..7 dequantise alternate weight stages, 8..11 and 12..15 fold (each
+// half of the activation rows), 16 copies weights, 18 activations, 17 and 19 issue MMAs.
 constexpr int kRowsThreads = 640;
 constexpr int kRowsFoldWarp0 = 8;
 constexpr int kRowsWeightWarp = 16;
@@ -100,9 +108,14 @@ constexpr int kRowsActWarp = 18;
 
 struct RowsSmem {
   std::uint64_t w_full[6], w_empty[6];
-  std::uint64_t b_full[6], b_empty[6];
-  std::uint64_t a_full[4], a_empty[4];
-  std::uint64_t d_full[2][4], d_free[2][4];  // [issuer][slot use]
+  std::uint64_t b_full[12];
+  std::uint64_t a_full[4];
+  // a group's MMAs have completed: its sums are in their slot, its A buffer and activations
+  // are free ([half of the activation rows at NT = 256][group modulo kR])
+  std::uint64_t done[2][8];
+  std::uint64_t d_free[2][4];
+  std::uint64_t set_bar[2];      // [fold set]
+  std::uint64_t res_full[2][2];  // [fold set][output buffer]: residual values have arrived
   std::uint32_t tmem_base;
   int abort_flag;
 };
@@ -120,6 +133,17 @@ struct Ring {
   }
 };
 
+// Waits of one warp on several barriers at once: every lane with `need` waits on its own
+// (a satisfied wait costs a warp on the order of two hundred cycles in this kernel, so they
+// are not made one after the other).  All lanes return the same value.
+__device__ __forceinline__ bool wait_lanes(bool need, std::uint64_t* bar, std::uint32_t parity,
+                                           volatile int* abort_flag) {
+  const bool ok = !need || tc_wait(bar, parity, abort_flag);
+  const bool all = __all_sync(0xffffffffu, ok);
+  __syncwarp();
+  return all;
+}
+
 // acc += {s, s} * {d0, d1}; volatile, so that it stays behind the wait for the tensor-memory
 // load that d0 and d1 come from.
 __device__ __forceinline__ void fma_f32x2(unsigned long long& acc, std::uint32_t d0, std::uint32_t d1,
@@ -135,6 +159,24 @@ __device__ __forceinline__ float hi_f(unsigned long long v) {
   return __uint_as_float(static_cast<std::uint32_t>(v >> 32));
 }
 
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, std::uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+// A barrier of the four warps of a fold set with the bounded wait of all others (a named
+// barrier would hang when one warp gives up).
+__device__ __forceinline__ bool fold_set_sync(std::uint64_t* bar, std::uint32_t& phase, int lane,
+                                              volatile int* abort_flag) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+  const bool ok = tc_wait(bar, phase, abort_flag);
+  phase ^= 1u;
+  return __all_sync(0xffffffffu, ok);
+}
+
 template <int NT, bool EXTRA>
 __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __grid_constant__ RowsParams p) {
   using C = RowsCfg<NT>;
@@ -144,27 +186,23 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
   RowsSmem* sm = reinterpret_cast<RowsSmem*>(smem);
   std::uint8_t* wst = smem + kRowsHeaderBytes;
   std::uint8_t* bst = wst + C::kW * kRowsWBytes;
+  std::uint8_t* outsm = bst + C::kB * C::kBoxBytes;
   volatile int* abort_flag = &sm->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
     for (int i = 0; i < C::kW; ++i) {
       mbar_init(&sm->w_full[i], 1);
-      mbar_init(&sm->w_empty[i], 8);  // once per dequantising warp
+      mbar_init(&sm->w_empty[i], 4);  // the warps of the stage's dequantising set
     }
-    for (int i = 0; i < C::kB; ++i) {
-      mbar_init(&sm->b_full[i], 1);
-      mbar_init(&sm->b_empty[i], C::kSub);
+    for (int i = 0; i < C::kB; ++i) mbar_init(&sm->b_full[i], 1);
+    for (int i = 0; i < C::kA; ++i) mbar_init(&sm->a_full[i], 4);
+    for (int h = 0; h < C::kSub; ++h) {
+      for (int i = 0; i < C::kR; ++i) mbar_init(&sm->done[h][i], 1);
+      for (int i = 0; i < C::kDB; ++i) mbar_init(&sm->d_free[h][i], C::kSub == 2 ? 4 : 8);
     }
-    for (int i = 0; i < C::kA; ++i) {
-      mbar_init(&sm->a_full[i], 4);
-      mbar_init(&sm->a_empty[i], C::kSub);
-    }
-    for (int h = 0; h < C::kSub; ++h)
-      for (int i = 0; i < C::kDB; ++i) {
-        mbar_init(&sm->d_full[h][i], 1);
-        mbar_init(&sm->d_free[h][i], C::kSub == 2 ? 4 : 8);
-      }
+    for (int i = 0; i < 2; ++i) mbar_init(&sm->set_bar[i], 4);
+    for (int i = 0; i < 4; ++i) mbar_init(&sm->res_full[i >> 1][i & 1], 1);
     sm->abort_flag = 0;
     mbar_init_fence();
   }
@@ -215,14 +253,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
             }
             std::uint8_t* st = wst + w.i * kRowsWBytes;
             mbar_arrive_expect_tx(&sm->w_full[w.i], kRowsWBytes);
-            for (int m = 0; m < (pair ? 2 : 1); ++m) {
-              asm volatile(
-                  "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-                  " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(st + m * (kRowsWBytes / 2))),
-                  "l"(m ? &L.tmap2 : &L.tmap), "r"(c * 32), "r"(j * (pair ? 64 : 128)),
-                  "r"(smem_u32(&sm->w_full[w.i]))
-                  : "memory");
-            }
+            for (int m = 0; m < (pair ? 2 : 1); ++m)
+              tma_load_2d(st + m * (kRowsWBytes / 2), m ? &L.tmap2 : &L.tmap, c * 32, j * (pair ? 64 : 128),
+                          &sm->w_full[w.i]);
             w.next(C::kW);
             if (w.i == 0) first_round = false;
           }
@@ -230,85 +263,86 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
         asm volatile("griddepcontrol.wait;" ::: "memory");
       }
     } else if (warp == kRowsActWarp) {
-      if (lane == 0) {
-        // ---------------- activations ----------------
-        Ring b;
-        bool first_round = true, ok = true;
-        for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
-          seek(u);
-          const RowsDesc& L = p.d[di];
-          const int t = (u - L.unit_begin) % L.tok_tiles;
-          const int G = L.K >> 7;
-          for (int g = 0; g < G; ++g) {
-            if (!first_round && !tc_wait(&sm->b_empty[b.i], b.phase ^ 1u, abort_flag)) {
-              ok = false;
-              break;
-            }
-            std::uint8_t* st = bst + b.i * C::kBBytes;
+      // ---------------- activations, half a group (64 k) at a time ----------------
+      Ring b;
+      int half = 0;  // halves so far
+      bool ok = true;
+      for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
+        seek(u);
+        const RowsDesc& L = p.d[di];
+        const int t = (u - L.unit_begin) % L.tok_tiles;
+        const int halves = L.K >> 6;
+        for (int q = 0; q < halves; ++q, ++half) {
+          // the group whose half was here is done with (by both issuers at NT = 256)
+          const std::uint32_t past = static_cast<std::uint32_t>(half - C::kB) >> 1;
+          ok = wait_lanes(half >= C::kB && lane < C::kSub, &sm->done[lane & (C::kSub - 1)][past % C::kR],
+                          (past / C::kR) & 1u, abort_flag);
+          if (!ok) break;
+          if (lane == 0) {
             // rows past M arrive as zeros
-            mbar_arrive_expect_tx(&sm->b_full[b.i], C::kBBytes);
-            for (int q = 0; q < 2; ++q) {
-              asm volatile(
-                  "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-                  " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(st + q * C::kBoxBytes)),
-                  "l"(&L.xmap), "r"(g * 128 + q * 64), "r"(t * NT), "r"(smem_u32(&sm->b_full[b.i]))
-                  : "memory");
-            }
-            b.next(C::kB);
-            if (b.i == 0) first_round = false;
+            mbar_arrive_expect_tx(&sm->b_full[b.i], C::kBoxBytes);
+            tma_load_2d(bst + b.i * C::kBoxBytes, &L.xmap, q * 64, t * NT, &sm->b_full[b.i]);
           }
+          b.next(C::kB);
         }
       }
-    } else if (warp == kRowsIssueWarp || C::kSub == 2) {
-      if (lane == 0) {
-        // ---------------- MMA issue ----------------
-        const int h = (warp - kRowsIssueWarp) >> 1;  // half of the activation rows (NT = 256)
-        const std::uint32_t desc_hi = static_cast<std::uint32_t>(tc_b_desc(0) >> 32);
-        const std::uint32_t desc_lo0 = static_cast<std::uint32_t>(tc_b_desc(0));
-        const std::uint32_t b0 = smem_u32(bst) + static_cast<std::uint32_t>(h) * 128u * 128u;
-        constexpr std::uint32_t kIdesc = tc_idesc(C::kSlot);
-        Ring a, b;
-        std::uint32_t git = 0;
-        int slot = h;  // NT = 256: slots go round over both halves, 2 git + h modulo 3
-        bool ok = true;
-        for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
-          seek(u);
-          const int G = p.d[di].K >> 7;
-          for (int g = 0; g < G; ++g, ++git) {
-            // The slot's previous sums have been read.  NT = 256: they were the other
-            // half's, three slot uses ago, i.e. of group git - 1 (h = 1) or git - 2 (h = 0);
-            // otherwise those of kD groups ago.
-            if (C::kSub == 2) {
-              const std::uint32_t back = h == 1 ? 1u : 2u;
-              if (git >= back)
-                ok = tc_wait(&sm->d_free[1 - h][(git - back) % C::kDB], ((git - back) / C::kDB) & 1u, abort_flag);
-            } else if (git >= C::kD) {
-              ok = tc_wait(&sm->d_free[0][git % C::kD], ((git / C::kD) - 1u) & 1u, abort_flag);
-            }
-            ok = ok && tc_wait(&sm->b_full[b.i], b.phase, abort_flag) &&
-                 tc_wait(&sm->a_full[a.i], a.phase, abort_flag);
-            if (!ok) break;
+    } else {
+      // ---------------- MMA issue ----------------
+      // NT = 256: one issuer per half of the activation rows; otherwise they take
+      // alternate groups, so that one's waits and commits run beside the other's MMAs.
+      const std::uint32_t who = static_cast<std::uint32_t>(warp - kRowsIssueWarp) >> 1;
+      const int h = C::kSub == 2 ? static_cast<int>(who) : 0;
+      const std::uint32_t desc_hi = static_cast<std::uint32_t>(tc_b_desc(0) >> 32);
+      const std::uint32_t desc_lo0 = static_cast<std::uint32_t>(tc_b_desc(0));
+      const std::uint32_t b0 = smem_u32(bst) + static_cast<std::uint32_t>(h) * 128u * 128u;
+      constexpr std::uint32_t kIdesc = tc_idesc(C::kSlot);
+      Ring b;
+      std::uint32_t git = 0;
+      int slot = h;  // NT = 256: slots go round over both halves, 2 git + h modulo 3
+      bool ok = true;
+      for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
+        seek(u);
+        const int G = p.d[di].K >> 7;
+        for (int g = 0; g < G; ++g, ++git) {
+          const Ring b_lo = b;
+          b.next(C::kB);
+          const Ring b_hi = b;
+          b.next(C::kB);
+          if (C::kSub == 1 && (git & 1u) != who) continue;
+          // Lane 0: the slot's previous sums have been read.  NT = 256: they were the other
+          // half's, three slot uses ago, i.e. of group git - 1 (h = 1) or git - 2 (h = 0);
+          // otherwise those of kD groups ago.  Lanes 1, 2: both halves of the group's
+          // activations have landed.  Lane 3: the A buffer holds the group.
+          const std::uint32_t back = C::kSub == 2 ? (h == 1 ? 1u : 2u) : static_cast<std::uint32_t>(C::kD);
+          const std::uint32_t prev = git - back;
+          std::uint64_t* bar = &sm->d_free[C::kSub == 2 ? 1 - h : 0][prev % C::kDB];
+          std::uint32_t parity = (prev / C::kDB) & 1u;
+          if (lane == 1) bar = &sm->b_full[b_lo.i], parity = b_lo.phase;
+          if (lane == 2) bar = &sm->b_full[b_hi.i], parity = b_hi.phase;
+          if (lane == 3) bar = &sm->a_full[git % C::kA], parity = (git / C::kA) & 1u;
+          ok = wait_lanes(lane < 4 && (lane > 0 || git >= back), bar, parity, abort_flag);
+          if (!ok) break;
+          if (lane == 0) {
             tc_fence_after();
-            const std::uint32_t b_addr = b0 + b.i * C::kBBytes;
-            tc_mma_group(tmem_d + slot * C::kSlot, tmem_a + a.i * 64,
-                         desc_lo0 | ((b_addr & 0x3FFFFu) >> 4), desc_hi, C::kBoxBytes >> 4, kIdesc);
-            tc_commit(&sm->d_full[h][git % C::kDB]);
-            tc_commit(&sm->a_empty[a.i]);
-            tc_commit(&sm->b_empty[b.i]);
-            a.next(C::kA);
-            b.next(C::kB);
-            slot += C::kSub;
-            if (slot >= C::kD) slot -= C::kD;
+            const std::uint32_t lo = (b0 + b_lo.i * C::kBoxBytes) >> 4, hi = (b0 + b_hi.i * C::kBoxBytes) >> 4;
+            const int s = C::kSub == 2 ? slot : static_cast<int>(git % C::kD);
+            tc_mma_group(tmem_d + s * C::kSlot, tmem_a + (git % C::kA) * 64, desc_lo0 | lo, desc_hi, hi - lo, kIdesc);
+            tc_commit(&sm->done[h][git % C::kR]);
           }
+          __syncwarp();
+          slot += 2;
+          if (slot >= C::kD) slot -= C::kD;
         }
       }
     }
   } else if (warp < kRowsFoldWarp0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegDequant) : "memory");
     // ---------------- dequantise: the A operand ----------------
-    const std::uint32_t set = warp >> 2;  // takes the groups of this parity
+    const int set = warp >> 2;  // takes the weight stages of this parity (kW is even)
     const int lrow = (warp & 3) * 32 + lane;
     const std::uint32_t a_base = tmem_a + (static_cast<std::uint32_t>((warp & 3) * 32) << 16);
+    // groups handed over at a time: both of a stage, except where there are only two buffers
+    constexpr int kStep = C::kA >= 4 ? 2 : 1;
     std::uint32_t git = 0;
     Ring w;
     bool alive = true;
@@ -318,44 +352,45 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
       // a pair's rows alternate gate, up (64 rows of either matrix)
       const bool pair = EXTRA && p.d[di].mode == kRowsPair;
       const int srow = pair ? (lrow & 1) * 64 + (lrow >> 1) : lrow;
-      for (int g = 0; g < G; ++g, ++git) {
-        if ((g & 1) == 0) {
-          const bool ok = tc_wait(&sm->w_full[w.i], w.phase, abort_flag);
-          alive = __all_sync(0xffffffffu, ok);
-          if (!alive) break;
-        }
-        if ((git & 1u) == set) {
-          const std::uint32_t buf = git % C::kA, use = git / C::kA;
-          if (use >= 1) {
-            const bool ok = tc_wait(&sm->a_empty[buf], (use - 1u) & 1u, abort_flag);
-            alive = __all_sync(0xffffffffu, ok);
-            if (!alive) break;
-          }
-          tc_fence_after();
+      for (int g = 0; g < G && alive; g += 2) {
+        const int n = G - g < 2 ? 1 : 2;
+        if ((w.i & 1) == set) {
           const std::uint8_t* rowp = wst + w.i * kRowsWBytes + srow * 128;
-          const std::uint32_t a_addr = a_base + buf * 64;
+          for (int i0 = 0; i0 < n; i0 += kStep) {
+            // lane 0: the stage has landed; the others: the groups that were in the A
+            // buffers are done with
+            const int m = n - i0 < kStep ? n - i0 : kStep;
+            const int which = (lane - 1) / C::kSub;  // group of this step the lane asks about
+            const std::uint32_t past = git + i0 + which - C::kA;
+            const bool asks = lane >= 1 && which < m && git + i0 + which >= static_cast<std::uint32_t>(C::kA);
+            alive = wait_lanes(lane == 0 || asks,
+                               lane == 0 ? &sm->w_full[w.i] : &sm->done[(lane - 1) & (C::kSub - 1)][past % C::kR],
+                               lane == 0 ? w.phase : (past / C::kR) & 1u, abort_flag);
+            if (!alive) break;
+            tc_fence_after();
+            for (int i = i0; i < i0 + m; ++i) {
+              const std::uint32_t a_addr = a_base + ((git + i) % C::kA) * 64;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            std::uint32_t regs[16];
-            const uint4 v = lds128(rowp + (((4 * (g & 1) + q) ^ (srow & 7)) << 4));
-            dequant_word_natural(v.x, regs);
-            dequant_word_natural(v.y, regs + 4);
-            dequant_word_natural(v.z, regs + 8);
-            dequant_word_natural(v.w, regs + 12);
-            tmem_st16(a_addr + 16 * q, regs);
+              for (int q = 0; q < 4; ++q) {
+                std::uint32_t regs[16];
+                const uint4 v = lds128(rowp + (((4 * i + q) ^ (srow & 7)) << 4));
+                dequant_word_natural(v.x, regs);
+                dequant_word_natural(v.y, regs + 4);
+                dequant_word_natural(v.z, regs + 8);
+                dequant_word_natural(v.w, regs + 12);
+                tmem_st16(a_addr + 16 * q, regs);
+              }
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane < m) mbar_arrive(&sm->a_full[(git + i0 + lane) % C::kA]);
           }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm->a_full[buf]);
-        }
-        if ((g & 1) || g == G - 1) {
-          // both sets have seen the stage's `full` phase and taken their group (if any)
-          // out of it
-          __syncwarp();
+          if (!alive) break;
           if (lane == 0) mbar_arrive(&sm->w_empty[w.i]);
-          w.next(C::kW);
         }
+        git += n;
+        w.next(C::kW);
       }
     }
   } else {
@@ -364,9 +399,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
     const int f = (warp - kRowsFoldWarp0) >> 2;  // half of the activation rows
     const int h = C::kSub == 2 ? f : 0;
     const int lrow = (warp & 3) * 32 + lane;
+    const bool leader = lrow == 0;  // issues the set's TMA stores
     const std::uint32_t d_base = tmem_d + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) +
                                  (C::kSub == 2 ? 0u : static_cast<std::uint32_t>(f) * C::kAcc);
+    std::uint8_t* outs = outsm + f * 2 * kRowsOutBytes;  // this set's two output buffers
+    constexpr int kChunks = C::kAcc / kRowsChunk;
     std::uint32_t git = 0;
+    std::uint32_t res_phase = 0;  // bit i: phase of res_full[f][i]
+    std::uint32_t set_phase = 0;
+    auto set_sync = [&] { return fold_set_sync(&sm->set_bar[f], set_phase, lane, abort_flag); };
     int slot = h;
     bool alive = true;
     for (int u = u_lo; u < u_hi && alive; ++u) {
@@ -375,9 +416,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
       const int N = L.N, G = L.K >> 7;
       const int j = (u - L.unit_begin) / L.tok_tiles, t = (u - L.unit_begin) - j * L.tok_tiles;
       const bool pair = EXTRA && L.mode == kRowsPair;
-      const int row = pair ? j * 64 + (lrow >> 1) : j * 128 + lrow;
+      const bool residual = EXTRA && L.mode == kRowsResidual;
+      const bool tma_residual = residual && !L.direct_store;
+      const int row0 = j * (pair ? 64 : 128);
+      const int row = row0 + (pair ? lrow >> 1 : lrow);
+      const int tok0 = t * NT + f * C::kAcc;
       const bool row_ok = row < N;
       const std::uint16_t* srow = ((pair && (lrow & 1)) ? L.S2 : L.S) + static_cast<std::size_t>(row_ok ? row : 0) * G;
+      auto fetch_residual = [&](int c) {
+        mbar_arrive_expect_tx(&sm->res_full[f][c & 1], kRowsOutBytes);
+        tma_load_2d(outs + (c & 1) * kRowsOutBytes, &L.rmap, row0, tok0 + c * kRowsChunk, &sm->res_full[f][c & 1]);
+      };
+      if (tma_residual && leader) {
+        // into the output buffers, once the previous unit's stores have read them
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        for (int c = 0; c < (kChunks < 2 ? kChunks : 2); ++c) fetch_residual(c);
+      }
       unsigned long long acc[C::kAcc / 2];
 #pragma unroll
       for (int n = 0; n < C::kAcc / 2; ++n) acc[n] = 0ull;
@@ -387,13 +441,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
         const std::uint32_t sc = __float_as_uint(__half2float(__ushort_as_half(sc_bits)));
         const unsigned long long s2 = (static_cast<unsigned long long>(sc) << 32) | sc;
         if (g + 1 < G) sc_bits = __ldg(srow + g + 1);
-        const std::uint32_t db = git % C::kDB;
-        const std::uint32_t use = git / C::kDB;
-        const bool ok = tc_wait(&sm->d_full[h][db], use & 1u, abort_flag);
+        const bool ok = tc_wait(&sm->done[h][git % C::kR], (git / C::kR) & 1u, abort_flag);
         alive = __all_sync(0xffffffffu, ok);
         if (!alive) break;
         tc_fence_after();
-        const std::uint32_t d_addr = d_base + slot * C::kSlot;
+        const std::uint32_t d_addr = d_base + (C::kSub == 2 ? slot : static_cast<int>(git % C::kD)) * C::kSlot;
 #pragma unroll
         for (int c = 0; c < C::kAcc / 32; ++c) {
           std::uint32_t d[32];
@@ -402,61 +454,94 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
             // the sums are in registers: hand the slot back before the arithmetic
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm->d_free[h][db]);
+            if (lane == 0) mbar_arrive(&sm->d_free[h][git % C::kDB]);
           }
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma_f32x2(acc[c * 16 + i], d[2 * i], d[2 * i + 1], s2);
         }
-        slot += C::kSub;
+        slot += 2;
         if (slot >= C::kD) slot -= C::kD;
       }
       if (!alive) break;
-      // ---- outputs: [activation row][weight row], a warp stores 32 consecutive rows ----
-      const int tok0 = t * NT + f * C::kAcc;
-      const int n_tok = L.M - tok0;  // may be negative: nothing to store
-      if (pair) {
-        // An even lane holds the gate and its odd neighbour the up output of one row: they
-        // exchange one of every two values, and each finishes one activation row.
-        std::uint16_t* yp = L.y + static_cast<std::size_t>(tok0 + (lane & 1)) * N + row;
+      // ---- outputs, 32 activation rows at a time through a box [activation row][weight
+      // row] in shared memory, which a TMA store (or the set's threads, where the TMA unit
+      // does not take the addresses) copies out ----
 #pragma unroll
-        for (int n = 0; n < C::kAcc; n += 2) {
-          const std::uint32_t mine = pack_bf16x2(lo_f(acc[n / 2]), hi_f(acc[n / 2]));
-          const std::uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
-          const std::uint16_t gate = static_cast<std::uint16_t>((lane & 1) ? other >> 16 : mine);
-          const std::uint16_t up = static_cast<std::uint16_t>((lane & 1) ? mine >> 16 : other);
-          if (row_ok && n + (lane & 1) < n_tok) {
+      for (int c = 0; c < kChunks; ++c) {
+        std::uint8_t* box = outs + (c & 1) * kRowsOutBytes;
+        if (tma_residual) {
+          const bool ok = tc_wait(&sm->res_full[f][c & 1], (res_phase >> (c & 1)) & 1u, abort_flag);
+          res_phase ^= 1u << (c & 1);
+          alive = __all_sync(0xffffffffu, ok);
+        } else {
+          if (leader) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          alive = set_sync();
+        }
+        if (!alive) break;
+        if (pair) {
+          // An even lane holds the gate and its odd neighbour the up output of one row: they
+          // exchange one of every two values, and each finishes one activation row.
+          std::uint8_t* slot16 = box + (lane & 1) * 128 + (lrow >> 1) * 2;
+#pragma unroll
+          for (int n = 0; n < kRowsChunk; n += 2) {
+            const unsigned long long v = acc[(c * kRowsChunk + n) / 2];
+            const std::uint32_t mine = pack_bf16x2(lo_f(v), hi_f(v));
+            const std::uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
+            const std::uint16_t gate = static_cast<std::uint16_t>((lane & 1) ? other >> 16 : mine);
+            const std::uint16_t up = static_cast<std::uint16_t>((lane & 1) ? mine >> 16 : other);
             // CUDALM's rounding order: bf16 after each projection, after silu, after the product
-            yp[static_cast<std::size_t>(n) * N] =
+            *reinterpret_cast<std::uint16_t*>(slot16 + n * 128) =
                 float_to_bf16_bits(bf16_bits_to_float(silu_bits(gate)) * bf16_bits_to_float(up));
           }
-        }
-      } else if (EXTRA && L.mode == kRowsResidual) {
-        std::uint16_t* yp = L.y + static_cast<std::size_t>(tok0) * N + row;
-        const std::uint16_t* rp = L.res + static_cast<std::size_t>(tok0) * N + row;
+        } else {
+          std::uint8_t* slot16 = box + lrow * 2;
 #pragma unroll
-        for (int c = 0; c < C::kAcc; c += 16) {
-          std::uint16_t r[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            r[i] = (row_ok && c + i < n_tok) ? rp[static_cast<std::size_t>(c + i) * N] : std::uint16_t{0};
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const unsigned long long v = acc[(c + i) / 2];
-            if (row_ok && c + i < n_tok)
-              yp[static_cast<std::size_t>(c + i) * N] =
-                  add_bits(r[i], float_to_bf16_bits((i & 1) ? hi_f(v) : lo_f(v)));
+          for (int n = 0; n < kRowsChunk; n += 2) {
+            const unsigned long long v = acc[(c * kRowsChunk + n) / 2];
+            std::uint32_t two = pack_bf16x2(lo_f(v), hi_f(v));
+            std::uint16_t* s0 = reinterpret_cast<std::uint16_t*>(slot16 + n * 256);
+            std::uint16_t* s1 = reinterpret_cast<std::uint16_t*>(slot16 + (n + 1) * 256);
+            if (tma_residual) {
+              *s0 = add_bits(*s0, static_cast<std::uint16_t>(two));
+              *s1 = add_bits(*s1, static_cast<std::uint16_t>(two >> 16));
+            } else {
+              *s0 = static_cast<std::uint16_t>(two);
+              *s1 = static_cast<std::uint16_t>(two >> 16);
+            }
           }
         }
-      } else {
-        std::uint16_t* yp = L.y + static_cast<std::size_t>(tok0) * N + row;
-#pragma unroll
-        for (int n = 0; n < C::kAcc; ++n) {
-          const unsigned long long v = acc[n / 2];
-          if (row_ok && n < n_tok)
-            yp[static_cast<std::size_t>(n) * N] = float_to_bf16_bits((n & 1) ? hi_f(v) : lo_f(v));
+        if (!L.direct_store) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        alive = set_sync();
+        if (!alive) break;
+        const int tok = tok0 + c * kRowsChunk;
+        if (!L.direct_store) {
+          if (leader && tok < L.M) {
+            asm volatile(
+                "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&L.ymap),
+                "r"(row0), "r"(tok), "r"(smem_u32(box))
+                : "memory");
+          }
+          if (leader) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          if (tma_residual && leader && c + 2 < kChunks) {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            fetch_residual(c + 2);
+          }
+        } else {
+          const int width = pair ? 64 : 128;
+          for (int i = lrow; i < kRowsChunk * width; i += 128) {
+            const int n = i / width, r = i - n * width;
+            if (tok + n >= L.M || row0 + r >= N) continue;
+            std::uint16_t v = *reinterpret_cast<const std::uint16_t*>(box + i * 2);
+            const std::size_t at = static_cast<std::size_t>(tok + n) * N + row0 + r;
+            if (residual) v = add_bits(L.res[at], v);
+            L.y[at] = v;
+          }
+          alive = set_sync();  // read before the box is written again
+          if (!alive) break;
         }
       }
     }
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   __syncthreads();
@@ -572,6 +657,12 @@ int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight
     d.K = l.K;
     d.M = l.M;
     d.mode = pair ? kRowsPair : (residual ? kRowsResidual : kRowsPlain);
+    d.direct_store = (l.N % 8 != 0 || !aligned_to(l.y, 16) || (residual && !aligned_to(residual, 16))) ? 1 : 0;
+    if (!d.direct_store) {
+      if (int rc = tc_encode(l.y, l.N, l.M, tile_rows, kRowsChunk, 2, &d.ymap)) return rc;
+      if (residual)
+        if (int rc = tc_encode(residual, l.N, l.M, tile_rows, kRowsChunk, 2, &d.rmap)) return rc;
+    }
     d.tok_tiles = (l.M + nt - 1) / nt;
     d.unit_begin = units;
     d.cost_begin = cost;
