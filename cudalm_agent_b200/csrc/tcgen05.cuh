@@ -17,6 +17,9 @@ constexpr unsigned long long kTcWaitNs = 400000000ull;
 // activations as bf16, 128-byte swizzle; 2: outputs as bf16, no swizzle.
 int tc_encode(const void* base, int inner, int outer, int box_inner, int box_outer, int kind,
               CUtensorMap* out);
+// Activations as bf16 [inner/64][outer][64], 128-byte swizzle, box `box_blocks` x `box_rows`
+// x 64: one copy brings several blocks of 64 k, each in the MMA's operand layout.
+int tc_encode_blocks(const void* base, int inner, int outer, int box_rows, int box_blocks, CUtensorMap* out);
 
 // ---------------------------------------------------------------------------
 // tcgen05 wrappers

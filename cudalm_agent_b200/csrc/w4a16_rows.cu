@@ -21,6 +21,14 @@
 // activations (shared memory, one group per stage) and A buffers / accumulator slots
 // (tensor memory).
 //
+// What bounds it: not DRAM (a projection is read once into L2) and not yet the tensor pipe
+// (a third busy): a chain of hand-overs per group.  An unsatisfied wait polls, and polling
+// slows every other role (with a tight loop in place of tc_wait's reads of the timer 6144 x
+// 1024 and 2048 rows took 40 us instead of 29); so each role waits once per group on all it
+// needs, and one barrier per group tells everybody that its MMAs are done.  2048 rows of a
+// layer with hidden size 1024 (four calls): 2018 us as passes of 64 rows, 180 with direct
+// stores and three commits per group, 145 now.
+//
 // Every wait is bounded; a wait that runs out raises a CTA-wide abort flag, the kernel
 // stores ERR_TIMEOUT in the status word, frees its tensor memory and returns.
 #include <cuda.h>
@@ -37,12 +45,9 @@ namespace {
 
 enum : int { kRowsPlain = 0, kRowsPair = 1, kRowsResidual = 2 };
 
-struct alignas(64) RowsDesc {
-  CUtensorMap tmap;   // weights as uint32 [N][K/8], box 128 rows (a pair: 64) x 32 words
-  CUtensorMap tmap2;  // kRowsPair: the second (up) matrix
-  CUtensorMap xmap;   // activations as bf16 [M][K], box NT rows x 64 values
-  CUtensorMap ymap;   // outputs as bf16 [M][N], box 32 rows x 128 values (a pair: 64)
-  CUtensorMap rmap;   // kRowsResidual: the residual, box as ymap
+// A launch's parameters reach each CTA through a cold constant cache, so the numbers that
+// every role needs before it can start lie together in front of the tensor maps.
+struct RowsInfo {
   const std::uint16_t* S;
   const std::uint16_t* S2;   // kRowsPair: scales of the second matrix
   const std::uint16_t* res;  // kRowsResidual: residual [M][N]; may be y
@@ -55,13 +60,20 @@ struct alignas(64) RowsDesc {
   int unit_end;
   int cost_begin;  // groups before this projection
 };
-
+struct alignas(64) RowsMaps {
+  CUtensorMap tmap;   // weights as uint32 [N][K/8], box 128 rows (a pair: 64) x 32 words
+  CUtensorMap tmap2;  // kRowsPair: the second (up) matrix
+  CUtensorMap xmap;   // activations as bf16 [K/64][M][64], box kBoxes x NT rows x 64 values
+  CUtensorMap ymap;   // outputs as bf16 [M][N], box 32 rows x 32 values (a pair: 16)
+  CUtensorMap rmap;   // kRowsResidual: the residual, box as ymap
+};
 struct RowsParams {
-  RowsDesc d[CUDALM_B200_MAX_INLINE_LINEARS];
   int n_desc;
   int total_units;
   int total_cost;
   int* status;
+  RowsInfo d[CUDALM_B200_MAX_INLINE_LINEARS];
+  RowsMaps maps[CUDALM_B200_MAX_INLINE_LINEARS];
 };
 
 // Register shares (of the 640 x 96 the CTA is launched with; 256 fold, 256 dequantising
@@ -72,30 +84,35 @@ struct RowsCfg {
   static constexpr int kSub = NT == 256 ? 2 : 1;         // MMAs along N per K=16 step (N <= 128 each)
   static constexpr int kSlot = NT / kSub;                // columns of an accumulator slot
   static constexpr int kAcc = NT / 2;                    // running sums per fold thread
+  static constexpr int kLd = 32;                         // columns read back at a time
   static constexpr int kD = NT == 256 ? 3 : (NT == 128 ? 2 : 4);  // accumulator slots
   // Barriers for a freed slot.  NT = 256: the three slots go round over both halves, so one
   // half can hold all three; four barriers keep it from lapping one.
   static constexpr int kDB = NT == 256 ? 4 : kD;
   static constexpr int kA = NT == 256 ? 2 : 4;           // A buffers of 64 columns
   static constexpr int kW = NT == 256 ? 2 : (NT == 128 ? 4 : 6);   // weight stages (two groups, 16 KB)
-  static constexpr int kB = NT == 256 ? 5 : (NT == 128 ? 8 : 12);  // activation stages (half a group)
+  // An activation stage holds kBoxes blocks of 64 k (two per group), fetched by one copy
+  // instruction: issuing one costs the copy thread several hundred cycles.
+  static constexpr int kBoxes = NT == 256 ? 1 : (NT == 128 ? 2 : 4);
+  static constexpr int kB = NT == 256 ? 5 : (NT == 128 ? 4 : 3);
   // Barriers for a finished group: more than any ring that waits for them reaches back.
   static constexpr int kR = NT == 256 ? 4 : 8;
   static constexpr int kBoxBytes = NT * 128;             // NT rows x 64 values
+  static constexpr int kBBytes = kBoxes * kBoxBytes;
   static constexpr int kRegFold = NT == 256 ? 176 : 136;
   static constexpr int kRegDequant = NT == 256 ? 48 : 72;
   static constexpr int kRegOther = NT == 256 ? 32 : 64;
   static_assert(kD * kSlot + kA * 64 <= 512, "tensor memory");
-  static_assert(kW % 2 == 0 && kA <= kR && kB / 2 < kR, "rings");
+  static_assert(kW % 2 == 0 && kA <= kR && kB * kBoxes / 2 < kR, "rings");
 };
 constexpr int kRowsWBytes = kTcRowsPerTile * 128;
 constexpr int kRowsHeaderBytes = 1024;
 constexpr int kRowsChunk = 32;                                       // activation rows per output box
-constexpr int kRowsOutBytes = kRowsChunk * kTcRowsPerTile * 2;       // two of them per fold set
+constexpr int kRowsOutBytes = kRowsChunk * 32 * 2;                   // two of them per fold warp
 template <int NT>
 constexpr int rows_smem_bytes() {
-  return 1024 + kRowsHeaderBytes + RowsCfg<NT>::kW * kRowsWBytes + RowsCfg<NT>::kB * RowsCfg<NT>::kBoxBytes +
-         4 * kRowsOutBytes;
+  return 1024 + kRowsHeaderBytes + RowsCfg<NT>::kW * kRowsWBytes + RowsCfg<NT>::kB * RowsCfg<NT>::kBBytes +
+         16 * kRowsOutBytes;
 }
 
 // Warp roles: 0..3 and 4..7 dequantise alternate weight stages, 8..11 and 12..15 fold (each
@@ -108,14 +125,13 @@ constexpr int kRowsActWarp = 18;
 
 struct RowsSmem {
   std::uint64_t w_full[6], w_empty[6];
-  std::uint64_t b_full[12];
+  std::uint64_t b_full[5];
   std::uint64_t a_full[4];
   // a group's MMAs have completed: its sums are in their slot, its A buffer and activations
   // are free ([half of the activation rows at NT = 256][group modulo kR])
   std::uint64_t done[2][8];
   std::uint64_t d_free[2][4];
-  std::uint64_t set_bar[2];      // [fold set]
-  std::uint64_t res_full[2][2];  // [fold set][output buffer]: residual values have arrived
+  std::uint64_t res_full[8][2];  // [fold warp][output buffer]: residual values have arrived
   std::uint32_t tmem_base;
   int abort_flag;
 };
@@ -159,6 +175,13 @@ __device__ __forceinline__ float hi_f(unsigned long long v) {
   return __uint_as_float(static_cast<std::uint32_t>(v >> 32));
 }
 
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, std::uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, std::uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -166,16 +189,33 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
-// A barrier of the four warps of a fold set with the bounded wait of all others (a named
-// barrier would hang when one warp gives up).
-__device__ __forceinline__ bool fold_set_sync(std::uint64_t* bar, std::uint32_t& phase, int lane,
-                                              volatile int* abort_flag) {
-  __syncwarp();
-  if (lane == 0) mbar_arrive(bar);
-  const bool ok = tc_wait(bar, phase, abort_flag);
-  phase ^= 1u;
-  return __all_sync(0xffffffffu, ok);
+// bf16(silu(gate)) of a bf16 value, the bits of silu_bits(): the approximate quotient (within
+// two units of the last of 24 bits; the denominator is kept inside its range) decides unless
+// it lies next to a rounding boundary of bf16, i.e. for all but one in 4,000 values.  The
+// correctly rounded division takes several times as long and was most of a pair's epilogue.
+__device__ __forceinline__ std::uint16_t silu_bits_near(std::uint16_t gate_bits) {
+  const float g = bf16_bits_to_float(gate_bits);
+  const float d = 1.0f + expf(-g);
+  const float q = __fdividef(g, d);
+  const int off = static_cast<int>(__float_as_uint(q) & 0xFFFFu) - 0x8000;
+  if (d < 1e30f && (off > 8 || off < -8)) return float_to_bf16_bits(q);
+  return silu_bits(gate_bits);
 }
+
+// The weight and activation tile of consecutive units of one projection.
+struct UnitTiles {
+  int j, t;
+  __device__ __forceinline__ void start(const RowsInfo& L, int u) {
+    j = (u - L.unit_begin) / L.tok_tiles;
+    t = (u - L.unit_begin) - j * L.tok_tiles;
+  }
+  __device__ __forceinline__ void next(const RowsInfo& L) {
+    if (++t == L.tok_tiles) {
+      t = 0;
+      ++j;
+    }
+  }
+};
 
 template <int NT, bool EXTRA>
 __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __grid_constant__ RowsParams p) {
@@ -186,7 +226,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
   RowsSmem* sm = reinterpret_cast<RowsSmem*>(smem);
   std::uint8_t* wst = smem + kRowsHeaderBytes;
   std::uint8_t* bst = wst + C::kW * kRowsWBytes;
-  std::uint8_t* outsm = bst + C::kB * C::kBoxBytes;
+  std::uint8_t* outsm = bst + C::kB * C::kBBytes;
   volatile int* abort_flag = &sm->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -201,8 +241,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
       for (int i = 0; i < C::kR; ++i) mbar_init(&sm->done[h][i], 1);
       for (int i = 0; i < C::kDB; ++i) mbar_init(&sm->d_free[h][i], C::kSub == 2 ? 4 : 8);
     }
-    for (int i = 0; i < 2; ++i) mbar_init(&sm->set_bar[i], 4);
-    for (int i = 0; i < 4; ++i) mbar_init(&sm->res_full[i >> 1][i & 1], 1);
+    if (EXTRA)
+      for (int i = 0; i < 16; ++i) mbar_init(&sm->res_full[i >> 1][i & 1], 1);
     sm->abort_flag = 0;
     mbar_init_fence();
   }
@@ -214,18 +254,35 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
   const std::uint32_t tmem_a = tmem_d + C::kD * C::kSlot;
 
   // This CTA's contiguous range of units: an equal share of the groups.
-  auto unit_at = [&](long long cost) -> int {
-    if (cost >= p.total_cost) return p.total_units;
-    int d = p.n_desc - 1;
-    while (d > 0 && p.d[d].cost_begin > cost) --d;
-    const int per = p.d[d].K >> 7;
-    return p.d[d].unit_begin + static_cast<int>((cost - p.d[d].cost_begin + per - 1) / per);
-  };
-  const int u_lo = unit_at(static_cast<long long>(blockIdx.x) * p.total_cost / gridDim.x);
-  const int u_hi = unit_at(static_cast<long long>(blockIdx.x + 1) * p.total_cost / gridDim.x);
+  // (One projection, as almost always: 32-bit arithmetic; 64-bit divisions by every thread
+  // took a microsecond.)
+  int u_lo, u_hi;
+  if (p.n_desc == 1 && p.total_units < (1 << 22)) {
+    const unsigned units = static_cast<unsigned>(p.total_units);
+    u_lo = static_cast<int>(blockIdx.x * units / gridDim.x);
+    u_hi = static_cast<int>((blockIdx.x + 1) * units / gridDim.x);
+  } else {
+    auto unit_at = [&](long long cost) -> int {
+      if (cost >= p.total_cost) return p.total_units;
+      int d = p.n_desc - 1;
+      while (d > 0 && p.d[d].cost_begin > cost) --d;
+      const int per = p.d[d].K >> 7;
+      return p.d[d].unit_begin + static_cast<int>((cost - p.d[d].cost_begin + per - 1) / per);
+    };
+    u_lo = unit_at(static_cast<long long>(blockIdx.x) * p.total_cost / gridDim.x);
+    u_hi = unit_at(static_cast<long long>(blockIdx.x + 1) * p.total_cost / gridDim.x);
+  }
   int di = 0;  // projection of the current unit
+  UnitTiles tile = {0, 0};
+  int tile_di = -1;
   auto seek = [&](int u) {
     while (u >= p.d[di].unit_end) ++di;
+    if (di != tile_di) {
+      tile_di = di;
+      tile.start(p.d[di], u);
+    } else {
+      tile.next(p.d[di]);
+    }
   };
 
   // Programmatic dependent launch: only the weight copies (weights are nobody's output)
@@ -242,9 +299,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
         bool first_round = true, ok = true;
         for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
           seek(u);
-          const RowsDesc& L = p.d[di];
+          const RowsInfo& L = p.d[di];
           const bool pair = EXTRA && L.mode == kRowsPair;
-          const int j = (u - L.unit_begin) / L.tok_tiles;
+          const int j = tile.j;
           const int stages = ((L.K >> 7) + 1) >> 1;
           for (int c = 0; c < stages; ++c) {
             if (!first_round && !tc_wait(&sm->w_empty[w.i], w.phase ^ 1u, abort_flag)) {
@@ -254,7 +311,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
             std::uint8_t* st = wst + w.i * kRowsWBytes;
             mbar_arrive_expect_tx(&sm->w_full[w.i], kRowsWBytes);
             for (int m = 0; m < (pair ? 2 : 1); ++m)
-              tma_load_2d(st + m * (kRowsWBytes / 2), m ? &L.tmap2 : &L.tmap, c * 32, j * (pair ? 64 : 128),
+              tma_load_2d(st + m * (kRowsWBytes / 2), m ? &p.maps[di].tmap2 : &p.maps[di].tmap, c * 32, j * (pair ? 64 : 128),
                           &sm->w_full[w.i]);
             w.next(C::kW);
             if (w.i == 0) first_round = false;
@@ -263,28 +320,40 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
         asm volatile("griddepcontrol.wait;" ::: "memory");
       }
     } else if (warp == kRowsActWarp) {
-      // ---------------- activations, half a group (64 k) at a time ----------------
+      // ---------------- activations ----------------
       Ring b;
-      int half = 0;  // halves so far
+      int n_stage = 0;  // stages so far
+      // last group (in the CTA's count) of the stages in the ring, to know when one is free
+      std::uint32_t last[C::kB];
+      std::uint32_t git = 0;
       bool ok = true;
       for (int u = u_lo; u < u_hi && ok && !*abort_flag; ++u) {
         seek(u);
-        const RowsDesc& L = p.d[di];
-        const int t = (u - L.unit_begin) % L.tok_tiles;
-        const int halves = L.K >> 6;
-        for (int q = 0; q < halves; ++q, ++half) {
-          // the group whose half was here is done with (by both issuers at NT = 256)
-          const std::uint32_t past = static_cast<std::uint32_t>(half - C::kB) >> 1;
-          ok = wait_lanes(half >= C::kB && lane < C::kSub, &sm->done[lane & (C::kSub - 1)][past % C::kR],
+        const RowsInfo& L = p.d[di];
+        const int t = tile.t;
+        const int blocks = L.K >> 6;
+        for (int q = 0; q < blocks; q += C::kBoxes, ++n_stage) {
+          // the last group whose activations were here is done with (by both issuers at
+          // NT = 256, where a stage is half a group)
+          std::uint32_t past = 0;
+#pragma unroll
+          for (int i = 0; i < C::kB; ++i)
+            if (i == b.i) past = last[i];
+          ok = wait_lanes(n_stage >= C::kB && lane < C::kSub, &sm->done[lane & (C::kSub - 1)][past % C::kR],
                           (past / C::kR) & 1u, abort_flag);
           if (!ok) break;
+          const int end = q + C::kBoxes < blocks ? q + C::kBoxes : blocks;
+#pragma unroll
+          for (int i = 0; i < C::kB; ++i)
+            if (i == b.i) last[i] = git + ((end - 1) >> 1);
           if (lane == 0) {
-            // rows past M arrive as zeros
-            mbar_arrive_expect_tx(&sm->b_full[b.i], C::kBoxBytes);
-            tma_load_2d(bst + b.i * C::kBoxBytes, &L.xmap, q * 64, t * NT, &sm->b_full[b.i]);
+            // rows past M and blocks past K arrive as zeros
+            mbar_arrive_expect_tx(&sm->b_full[b.i], C::kBBytes);
+            tma_load_3d(bst + b.i * C::kBBytes, &p.maps[di].xmap, 0, t * NT, q, &sm->b_full[b.i]);
           }
           b.next(C::kB);
         }
+        git += blocks >> 1;
       }
     } else {
       // ---------------- MMA issue ----------------
@@ -304,10 +373,12 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
         seek(u);
         const int G = p.d[di].K >> 7;
         for (int g = 0; g < G; ++g, ++git) {
+          // the stage or stages of the group, and where in them its two blocks of 64 k are
           const Ring b_lo = b;
-          b.next(C::kB);
+          if (C::kBoxes == 1) b.next(C::kB);
           const Ring b_hi = b;
-          b.next(C::kB);
+          const std::uint32_t block = C::kBoxes == 4 ? 2u * (g & 1) : 0u;
+          if (C::kBoxes <= 2 || (g & 1) || g == G - 1) b.next(C::kB);
           if (C::kSub == 1 && (git & 1u) != who) continue;
           // Lane 0: the slot's previous sums have been read.  NT = 256: they were the other
           // half's, three slot uses ago, i.e. of group git - 1 (h = 1) or git - 2 (h = 0);
@@ -324,7 +395,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
           if (!ok) break;
           if (lane == 0) {
             tc_fence_after();
-            const std::uint32_t lo = (b0 + b_lo.i * C::kBoxBytes) >> 4, hi = (b0 + b_hi.i * C::kBoxBytes) >> 4;
+            const std::uint32_t lo = (b0 + b_lo.i * C::kBBytes + block * C::kBoxBytes) >> 4;
+            const std::uint32_t hi =
+                C::kBoxes == 1 ? (b0 + b_hi.i * C::kBBytes) >> 4 : lo + (C::kBoxBytes >> 4);
             const int s = C::kSub == 2 ? slot : static_cast<int>(git % C::kD);
             tc_mma_group(tmem_d + s * C::kSlot, tmem_a + (git % C::kA) * 64, desc_lo0 | lo, desc_hi, hi - lo, kIdesc);
             tc_commit(&sm->done[h][git % C::kR]);
@@ -341,8 +414,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
     const int set = warp >> 2;  // takes the weight stages of this parity (kW is even)
     const int lrow = (warp & 3) * 32 + lane;
     const std::uint32_t a_base = tmem_a + (static_cast<std::uint32_t>((warp & 3) * 32) << 16);
-    // groups handed over at a time: both of a stage, except where there are only two buffers
-    constexpr int kStep = C::kA >= 4 ? 2 : 1;
+    // groups handed over at a time: both of a stage where a group is short (NT = 64)
+    constexpr int kStep = NT == 64 ? 2 : 1;
     std::uint32_t git = 0;
     Ring w;
     bool alive = true;
@@ -399,35 +472,38 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
     const int f = (warp - kRowsFoldWarp0) >> 2;  // half of the activation rows
     const int h = C::kSub == 2 ? f : 0;
     const int lrow = (warp & 3) * 32 + lane;
-    const bool leader = lrow == 0;  // issues the set's TMA stores
     const std::uint32_t d_base = tmem_d + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) +
                                  (C::kSub == 2 ? 0u : static_cast<std::uint32_t>(f) * C::kAcc);
-    std::uint8_t* outs = outsm + f * 2 * kRowsOutBytes;  // this set's two output buffers
+    const int fw = warp - kRowsFoldWarp0;
+    std::uint8_t* outs = outsm + fw * 2 * kRowsOutBytes;  // this warp's two output buffers
     constexpr int kChunks = C::kAcc / kRowsChunk;
+    static_assert(kChunks == 1 || kChunks % 2 == 0, "output buffers");
     std::uint32_t git = 0;
-    std::uint32_t res_phase = 0;  // bit i: phase of res_full[f][i]
-    std::uint32_t set_phase = 0;
-    auto set_sync = [&] { return fold_set_sync(&sm->set_bar[f], set_phase, lane, abort_flag); };
+    std::uint32_t res_phase = 0;  // bit i: phase of res_full[fw][i]
     int slot = h;
     bool alive = true;
     for (int u = u_lo; u < u_hi && alive; ++u) {
       seek(u);
-      const RowsDesc& L = p.d[di];
+      const RowsInfo& L = p.d[di];
       const int N = L.N, G = L.K >> 7;
-      const int j = (u - L.unit_begin) / L.tok_tiles, t = (u - L.unit_begin) - j * L.tok_tiles;
-      const bool pair = EXTRA && L.mode == kRowsPair;
+      const int j = tile.j, t = tile.t;
+      const bool pair = EXTRA && NT < 256 && L.mode == kRowsPair;
       const bool residual = EXTRA && L.mode == kRowsResidual;
       const bool tma_residual = residual && !L.direct_store;
-      const int row0 = j * (pair ? 64 : 128);
-      const int row = row0 + (pair ? lrow >> 1 : lrow);
+      // first weight row of this warp, and this lane's (a pair: lanes alternate gate, up)
+      const int row0 = pair ? j * 64 + (warp & 3) * 16 : j * 128 + (warp & 3) * 32;
+      const int row = row0 + (pair ? lane >> 1 : lane);
       const int tok0 = t * NT + f * C::kAcc;
       const bool row_ok = row < N;
       const std::uint16_t* srow = ((pair && (lrow & 1)) ? L.S2 : L.S) + static_cast<std::size_t>(row_ok ? row : 0) * G;
+      // the buffers take turns, across units too (at NT = 64 a unit has one box only)
+      auto buffer = [&](int c) { return kChunks == 1 ? (u - u_lo) & 1 : c & 1; };
       auto fetch_residual = [&](int c) {
-        mbar_arrive_expect_tx(&sm->res_full[f][c & 1], kRowsOutBytes);
-        tma_load_2d(outs + (c & 1) * kRowsOutBytes, &L.rmap, row0, tok0 + c * kRowsChunk, &sm->res_full[f][c & 1]);
+        const int b = buffer(c);
+        mbar_arrive_expect_tx(&sm->res_full[fw][b], kRowsOutBytes);
+        tma_load_2d(outs + b * kRowsOutBytes, &p.maps[di].rmap, row0, tok0 + c * kRowsChunk, &sm->res_full[fw][b]);
       };
-      if (tma_residual && leader) {
+      if (tma_residual && lane == 0) {
         // into the output buffers, once the previous unit's stores have read them
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         for (int c = 0; c < (kChunks < 2 ? kChunks : 2); ++c) fetch_residual(c);
@@ -447,60 +523,78 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
         tc_fence_after();
         const std::uint32_t d_addr = d_base + (C::kSub == 2 ? slot : static_cast<int>(git % C::kD)) * C::kSlot;
 #pragma unroll
-        for (int c = 0; c < C::kAcc / 32; ++c) {
-          std::uint32_t d[32];
-          tmem_ld_cols<32>(d_addr + c * 32, d);
-          if (c == C::kAcc / 32 - 1) {
+        for (int c = 0; c < C::kAcc / C::kLd; ++c) {
+          std::uint32_t d[C::kLd];
+          tmem_ld_cols<C::kLd>(d_addr + c * C::kLd, d);
+          if (c == C::kAcc / C::kLd - 1) {
             // the sums are in registers: hand the slot back before the arithmetic
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm->d_free[h][git % C::kDB]);
           }
 #pragma unroll
-          for (int i = 0; i < 16; ++i) fma_f32x2(acc[c * 16 + i], d[2 * i], d[2 * i + 1], s2);
+          for (int i = 0; i < C::kLd / 2; ++i)
+            fma_f32x2(acc[c * (C::kLd / 2) + i], d[2 * i], d[2 * i + 1], s2);
         }
         slot += 2;
         if (slot >= C::kD) slot -= C::kD;
       }
       if (!alive) break;
-      // ---- outputs, 32 activation rows at a time through a box [activation row][weight
-      // row] in shared memory, which a TMA store (or the set's threads, where the TMA unit
-      // does not take the addresses) copies out ----
+      // ---- outputs, 32 activation rows at a time through the warp's own box [activation
+      // row][weight row] in shared memory, which a TMA store (or the lanes, where the TMA
+      // unit does not take the addresses) copies out.  Boxes of all four warps together
+      // make longer rows, but their two barriers per box cost more than the stores. ----
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
-        std::uint8_t* box = outs + (c & 1) * kRowsOutBytes;
+        const int b = buffer(c);
+        std::uint8_t* box = outs + b * kRowsOutBytes;
         if (tma_residual) {
-          const bool ok = tc_wait(&sm->res_full[f][c & 1], (res_phase >> (c & 1)) & 1u, abort_flag);
-          res_phase ^= 1u << (c & 1);
+          const bool ok = tc_wait(&sm->res_full[fw][b], (res_phase >> b) & 1u, abort_flag);
+          res_phase ^= 1u << b;
           alive = __all_sync(0xffffffffu, ok);
+          if (!alive) break;
         } else {
-          if (leader) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          alive = set_sync();
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
         }
-        if (!alive) break;
         if (pair) {
           // An even lane holds the gate and its odd neighbour the up output of one row: they
-          // exchange one of every two values, and each finishes one activation row.
-          std::uint8_t* slot16 = box + (lane & 1) * 128 + (lrow >> 1) * 2;
+          // exchange one of every two values, and each finishes one activation row.  The
+          // box first takes {gate, up} words and is then rewritten from the front, eight
+          // words a lane at a time (all of a thread's values unrolled: 71.6 us against 68.8
+          // for 3584 x 1024 and 2048 rows).
+          std::uint32_t* words = reinterpret_cast<std::uint32_t*>(box) + lane;
 #pragma unroll
           for (int n = 0; n < kRowsChunk; n += 2) {
             const unsigned long long v = acc[(c * kRowsChunk + n) / 2];
             const std::uint32_t mine = pack_bf16x2(lo_f(v), hi_f(v));
             const std::uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            const std::uint16_t gate = static_cast<std::uint16_t>((lane & 1) ? other >> 16 : mine);
-            const std::uint16_t up = static_cast<std::uint16_t>((lane & 1) ? mine >> 16 : other);
-            // CUDALM's rounding order: bf16 after each projection, after silu, after the product
-            *reinterpret_cast<std::uint16_t*>(slot16 + n * 128) =
-                float_to_bf16_bits(bf16_bits_to_float(silu_bits(gate)) * bf16_bits_to_float(up));
+            words[n * 16] = (lane & 1) ? __byte_perm(mine, other, 0x3276) : __byte_perm(mine, other, 0x5410);
+          }
+          std::uint8_t* slot16 = box + (lane & 1) * 32 + (lane >> 1) * 2;
+#pragma unroll 1
+          for (int i = 0; i < kRowsChunk / 2; i += 8) {
+            std::uint32_t w[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = words[(i + k) * 32];
+            __syncwarp();  // the words behind these outputs have been read by every lane
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              // CUDALM's rounding order: bf16 after each projection, after silu, after the product
+              const float silu = bf16_bits_to_float(silu_bits_near(static_cast<std::uint16_t>(w[k])));
+              *reinterpret_cast<std::uint16_t*>(slot16 + (i + k) * 64) =
+                  float_to_bf16_bits(silu * bf16_bits_to_float(static_cast<std::uint16_t>(w[k] >> 16)));
+            }
+            __syncwarp();
           }
         } else {
-          std::uint8_t* slot16 = box + lrow * 2;
+          std::uint8_t* slot16 = box + lane * 2;
 #pragma unroll
           for (int n = 0; n < kRowsChunk; n += 2) {
             const unsigned long long v = acc[(c * kRowsChunk + n) / 2];
-            std::uint32_t two = pack_bf16x2(lo_f(v), hi_f(v));
-            std::uint16_t* s0 = reinterpret_cast<std::uint16_t*>(slot16 + n * 256);
-            std::uint16_t* s1 = reinterpret_cast<std::uint16_t*>(slot16 + (n + 1) * 256);
+            const std::uint32_t two = pack_bf16x2(lo_f(v), hi_f(v));
+            std::uint16_t* s0 = reinterpret_cast<std::uint16_t*>(slot16 + n * 64);
+            std::uint16_t* s1 = reinterpret_cast<std::uint16_t*>(slot16 + (n + 1) * 64);
             if (tma_residual) {
               *s0 = add_bits(*s0, static_cast<std::uint16_t>(two));
               *s1 = add_bits(*s1, static_cast<std::uint16_t>(two >> 16));
@@ -510,34 +604,33 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
             }
           }
         }
-        if (!L.direct_store) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        alive = set_sync();
-        if (!alive) break;
         const int tok = tok0 + c * kRowsChunk;
         if (!L.direct_store) {
-          if (leader && tok < L.M) {
-            asm volatile(
-                "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&L.ymap),
-                "r"(row0), "r"(tok), "r"(smem_u32(box))
-                : "memory");
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            if (tok < L.M && row0 < N)
+              asm volatile(
+                  "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                      &p.maps[di].ymap),
+                  "r"(row0), "r"(tok), "r"(smem_u32(box))
+                  : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            if (tma_residual && c + 2 < kChunks) {
+              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              fetch_residual(c + 2);
+            }
           }
-          if (leader) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          if (tma_residual && leader && c + 2 < kChunks) {
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            fetch_residual(c + 2);
-          }
-        } else {
-          const int width = pair ? 64 : 128;
-          for (int i = lrow; i < kRowsChunk * width; i += 128) {
-            const int n = i / width, r = i - n * width;
-            if (tok + n >= L.M || row0 + r >= N) continue;
-            std::uint16_t v = *reinterpret_cast<const std::uint16_t*>(box + i * 2);
-            const std::size_t at = static_cast<std::size_t>(tok + n) * N + row0 + r;
+        } else if (row_ok) {
+          // each lane copies out the values it has written
+          const int step = pair ? 2 : 1, n0 = pair ? lane & 1 : 0;
+          for (int n = n0; n < kRowsChunk && tok + n < L.M; n += step) {
+            std::uint16_t v = *reinterpret_cast<const std::uint16_t*>(
+                pair ? box + n * 32 + (lane >> 1) * 2 : box + n * 64 + lane * 2);
+            const std::size_t at = static_cast<std::size_t>(tok + n) * N + row;
             if (residual) v = add_bits(L.res[at], v);
             L.y[at] = v;
           }
-          alive = set_sync();  // read before the box is written again
-          if (!alive) break;
         }
       }
     }
@@ -615,27 +708,32 @@ int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight
   for (int i = 0; i < count; ++i)
     if (!rows_eligible(ls[i])) return CUDALM_B200_ERR_UNSUPPORTED;
   const int tile_rows = pair ? 64 : 128;
-  // The tile that finishes first: the most loaded SM's groups times what a group costs
-  // with that many activation rows.
+  // The tile that finishes first: units of the most loaded SM times a unit's cycles, which
+  // are its groups' and a fixed part (filling the pipeline, outputs).  Measured on 1024 x
+  // 3584 and 6144 x 1024 with 2048 rows, 256 / 128 / 64: 29.3 / 19.8 / 34.4 and 29.4 / 34.9 /
+  // 54.2 us.  A pair's silu lengthens the fixed part; with 128 sums a thread it has no
+  // registers (3584 x 1024, 2048 rows: 140 us against 70 and 78).
   static constexpr int kTiles[3] = {256, 128, 64};
-  static constexpr int kCycles[3] = {1150, 650, 420};
+  static constexpr int kPerGroup[3] = {1560, 1075, 965};
+  static constexpr int kPerUnit[3] = {6000, 2400, 1600};
+  static constexpr int kPerPair[3] = {0, 10300, 3700};
   int nt = 0;
   long long best = 0;
-  for (int k = 0; k < 3; ++k) {
-    long long groups = 0, units = 0, longest = 0;
+  for (int k = pair ? 1 : 0; k < 3; ++k) {
+    long long cycles = 0, units = 0, groups = 0, longest = 0;
     for (int i = 0; i < count; ++i) {
       const long long n = static_cast<long long>((ls[i].N + tile_rows - 1) / tile_rows) *
                           ((ls[i].M + kTiles[k] - 1) / kTiles[k]);
+      const long long unit = static_cast<long long>(ls[i].K >> 7) * kPerGroup[k] + (pair ? kPerPair : kPerUnit)[k];
       units += n;
       groups += n * (ls[i].K >> 7);
-      if ((ls[i].K >> 7) > longest) longest = ls[i].K >> 7;
+      cycles += n * unit;
+      if (unit > longest) longest = unit;
     }
     if (units > 0x3fffffff || groups > 0x3fffffff) return CUDALM_B200_ERR_TOO_LARGE;
-    const long long rounds = (units + num_sms() - 1) / num_sms();
-    long long load = count == 1 ? rounds * longest : (groups + num_sms() - 1) / num_sms() + longest / 2;
-    if (load < longest) load = longest;
-    if (nt == 0 || load * kCycles[k] < best) {
-      best = load * kCycles[k];
+    const long long time = count == 1 ? (units + num_sms() - 1) / num_sms() * longest : cycles / num_sms() + longest;
+    if (nt == 0 || time < best) {
+      best = time;
       nt = kTiles[k];
     }
   }
@@ -644,11 +742,12 @@ int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight
   int units = 0, cost = 0;
   for (int i = 0; i < count; ++i) {
     const cudalm_b200_linear& l = ls[i];
-    RowsDesc& d = p.d[i];
-    if (int rc = tc_encode(l.weight, l.K / 8, l.N, 32, tile_rows, 0, &d.tmap)) return rc;
+    RowsInfo& d = p.d[i];
+    RowsMaps& maps = p.maps[i];
+    if (int rc = tc_encode(l.weight, l.K / 8, l.N, 32, tile_rows, 0, &maps.tmap)) return rc;
     if (pair)
-      if (int rc = tc_encode(weight2, l.K / 8, l.N, 32, tile_rows, 0, &d.tmap2)) return rc;
-    if (int rc = tc_encode(l.x, l.K, l.M, 64, nt, 1, &d.xmap)) return rc;
+      if (int rc = tc_encode(weight2, l.K / 8, l.N, 32, tile_rows, 0, &maps.tmap2)) return rc;
+    if (int rc = tc_encode_blocks(l.x, l.K, l.M, nt, nt == 256 ? 1 : (nt == 128 ? 2 : 4), &maps.xmap)) return rc;
     d.S = l.scales;
     d.S2 = scales2;
     d.res = residual;
@@ -659,9 +758,9 @@ int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight
     d.mode = pair ? kRowsPair : (residual ? kRowsResidual : kRowsPlain);
     d.direct_store = (l.N % 8 != 0 || !aligned_to(l.y, 16) || (residual && !aligned_to(residual, 16))) ? 1 : 0;
     if (!d.direct_store) {
-      if (int rc = tc_encode(l.y, l.N, l.M, tile_rows, kRowsChunk, 2, &d.ymap)) return rc;
+      if (int rc = tc_encode(l.y, l.N, l.M, tile_rows / 4, kRowsChunk, 2, &maps.ymap)) return rc;
       if (residual)
-        if (int rc = tc_encode(residual, l.N, l.M, tile_rows, kRowsChunk, 2, &d.rmap)) return rc;
+        if (int rc = tc_encode(residual, l.N, l.M, tile_rows / 4, kRowsChunk, 2, &maps.rmap)) return rc;
     }
     d.tok_tiles = (l.M + nt - 1) / nt;
     d.unit_begin = units;

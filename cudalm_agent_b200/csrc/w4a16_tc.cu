@@ -830,8 +830,6 @@ constexpr int kTcMapCache = 1024;
 
 int tc_encode(const void* base, int inner, int outer, int box_inner, int box_outer, int kind,
               CUtensorMap* out) {
-  // kind 0: packed weights as uint32, 128-byte swizzle; 1: activations as bf16, 128-byte
-  // swizzle; 2: outputs as bf16, no swizzle
   static std::mutex mu;
   static TcMapEntry cache[kTcMapCache];
   const std::uintptr_t h = reinterpret_cast<std::uintptr_t>(base);
@@ -851,12 +849,17 @@ int tc_encode(const void* base, int inner, int outer, int box_inner, int box_out
   EncodeTiledFn fn = tc_encode_fn();
   if (!fn) return CUDALM_B200_ERR_CUDA;
   const int esize = kind == 0 ? 4 : 2;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(inner) * esize};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer)};
-  const cuuint32_t elem[2] = {1, 1};
+  // kind 3: [inner/64][outer][64] with a box of `box_inner` x `box_outer` x 64
+  const bool blocks = kind == 3;
+  const cuuint64_t pitch = static_cast<cuuint64_t>(inner) * esize;
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(blocks ? 64 : inner), static_cast<cuuint64_t>(outer),
+                              static_cast<cuuint64_t>(inner / 64)};
+  const cuuint64_t strides[2] = {pitch, 128};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(blocks ? 64 : box_inner), static_cast<cuuint32_t>(box_outer),
+                             static_cast<cuuint32_t>(box_inner)};
+  const cuuint32_t elem[3] = {1, 1, 1};
   const CUresult r =
-      fn(out, kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2,
+      fn(out, kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, blocks ? 3 : 2,
          const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
          kind == 2 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -868,6 +871,10 @@ int tc_encode(const void* base, int inner, int outer, int box_inner, int box_out
   cache[slot].key = TcMapKey{base, inner, outer, box_inner, box_outer, kind};
   cache[slot].map = *out;
   return CUDALM_B200_OK;
+}
+
+int tc_encode_blocks(const void* base, int inner, int outer, int box_rows, int box_blocks, CUtensorMap* out) {
+  return tc_encode(base, inner, outer, box_blocks, box_rows, 3, out);
 }
 
 namespace {
