@@ -1,5 +1,5 @@
-// Lean W4A16 kernel for single calls of a few megabytes with up to 8 activation
-// rows: the form in which a decode step calls cudalm::int4_gemv_bf16 (one
+// Lean W4A16 kernel for single calls of a few megabytes with few activation rows
+// (to 16; to 64 where a long K meets few weight rows): the form in which a decode step calls cudalm::int4_gemv_bf16 (one
 // projection per launch, each depending on the one before).
 //
 // Such a call moves 0.3 - 3 MB, i.e. well under a microsecond of HBM time, so
@@ -19,8 +19,8 @@
 //     by every warp of the SM);
 //   * the 4-bit values become exact bf16 integers (one LOP3 and one packed
 //     subtraction per two values) and go through mma.sync m16n8k16 with the 16
-//     weight rows as the A operand and the activation rows as the 8 columns, eight
-//     MMAs per group, then acc += scale * group_sum in fp32.  Products are exact,
+//     weight rows as the A operand and the activation rows as the columns (tiles of 8), eight
+//     MMAs per group and tile, then acc += scale * group_sum in fp32.  Products are exact,
 //     sums are fp32, activations are used as they are (any finite or non-finite
 //     value), and a group of zero nibbles contributes an exact zero;
 //   * the warps' partial sums meet in 4 KB of shared memory and are added in the
@@ -42,7 +42,7 @@ namespace cb200 {
 constexpr int kDirectWarps = 8;
 constexpr int kDirectThreads = kDirectWarps * 32;
 constexpr int kDirectBatch = 4;     // groups whose weights a lane holds in registers at once
-constexpr int kDirectMaxRows = 16;  // activation rows: one or two MMA column tiles of 8
+constexpr int kDirectMaxRows = 64;  // activation rows: one to eight MMA column tiles of 8
 
 enum : int { kDirectPlain = 0, kDirectPair = 1, kDirectResidual = 2 };
 
@@ -137,11 +137,51 @@ __device__ __forceinline__ void direct_group(const uint4& qa, const uint4& qb,
     for (int i = 0; i < 4; ++i) sum[n][i] = c0[n][i] + c1[n][i];
 }
 
+// The same for four or eight column tiles: the activations of one weight word at a time, the
+// next word's requested before this one's MMAs.
+template <int NCOL>
+__device__ __forceinline__ void direct_group_wide(const uint4& qa, const uint4& qb,
+                                                  const std::uint16_t* const (&xr)[NCOL],
+                                                  const bool (&x_real)[NCOL], int x_off, float (&sum)[NCOL][4]) {
+  const std::uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w};
+  const std::uint32_t wb[4] = {qb.x, qb.y, qb.z, qb.w};
+  uint4 X[2][NCOL];
+  auto load = [&](int w) {
+#pragma unroll
+    for (int n = 0; n < NCOL; ++n)
+      X[w & 1][n] = x_real[n] ? ldg_activations(xr[n] + x_off + w * 8) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  load(0);
+#pragma unroll
+  for (int n = 0; n < NCOL; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[n][i] = 0.f;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    if (w < 3) load(w + 1);
+    std::uint32_t A[4], B[4];
+    dequant_pairs(wa[w], A);
+    dequant_pairs(wb[w], B);
+#pragma unroll
+    for (int n = 0; n < NCOL; ++n) {
+      const uint4& v = X[w & 1][n];
+      mma_m16n8k16_bf16(sum[n], A[0], B[0], A[1], B[1], __byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632));
+    }
+#pragma unroll
+    for (int n = 0; n < NCOL; ++n) {
+      const uint4& v = X[w & 1][n];
+      mma_m16n8k16_bf16(sum[n], A[2], B[2], A[3], B[3], __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
+    }
+  }
+}
+
 // NCOL: tiles of 8 activation rows.
 template <int NCOL>
-__global__ void __launch_bounds__(kDirectThreads, NCOL == 1 ? 3 : 2)
+__global__ void __launch_bounds__(kDirectThreads, NCOL == 1 ? 3 : (NCOL == 2 ? 2 : 1))
 w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
-  __shared__ float4 red[2][NCOL][kDirectWarps][32];
+  // (eight column tiles: 32 KB for one matrix; a pair's second sums follow in a second round)
+  constexpr int kMats = NCOL == 8 ? 1 : 2;
+  __shared__ float4 red[kMats][NCOL][kDirectWarps][32];
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
@@ -211,7 +251,8 @@ w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
         const int g = g0 + (pair ? (j & (kDirectBatch / 2 - 1)) : j);
         if (g < gend) {
           float sum[NCOL][4];
-          direct_group<NCOL>(qa[j], qb[j], xr, x_real, g * 128, sum);
+          if (NCOL <= 2) direct_group<NCOL>(qa[j], qb[j], xr, x_real, g * 128, sum);
+          else direct_group_wide<NCOL>(qa[j], qb[j], xr, x_real, g * 128, sum);
           const float s_lo = __half2float(__ushort_as_half(sca[j]));
           const float s_hi = __half2float(__ushort_as_half(scb[j]));
 #pragma unroll
@@ -231,29 +272,46 @@ w4a16_direct_kernel(const __grid_constant__ DirectParams p) {
 #pragma unroll
   for (int n = 0; n < NCOL; ++n) {
     red[0][n][warp][lane] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
-    if (pair) red[1][n][warp][lane] = make_float4(acc2[n][0], acc2[n][1], acc2[n][2], acc2[n][3]);
+    if (pair && kMats == 2) red[kMats - 1][n][warp][lane] = make_float4(acc2[n][0], acc2[n][1], acc2[n][2], acc2[n][3]);
   }
   __syncthreads();
 
   // Outputs of the CTA's m-tiles: (row r, activation row 8 n + c) of a tile sits in lane
   // (r % 8) * 4 + c / 2, element (r / 8) * 2 + c % 2 of each of the tile's warps.
+  constexpr int kOut = kDirectWarps * 128 * NCOL / kDirectThreads;  // most outputs per thread
   const int n_out = d.tiles_per_cta * 128 * NCOL;
-  for (int idx = tid; idx < n_out; idx += kDirectThreads) {
+  auto total = [&](int mat, int idx) {
+    const int r = idx & 15, c = (idx >> 4) & 7, n = (idx >> 7) % NCOL, tile = (idx >> 7) / NCOL;
+    const int src_lane = (r & 7) * 4 + (c >> 1), elem = (r >> 3) * 2 + (c & 1), w0 = tile * nsplit;
+    float v = 0.f;
+    for (int s = 0; s < nsplit; ++s) v += reinterpret_cast<const float*>(&red[mat][n][w0 + s][src_lane])[elem];
+    return v;
+  };
+  std::uint16_t gate_bits[kMats == 1 ? kOut : 1];
+  if (kMats == 1 && pair) {
+    // the gate sums first, then the up sums through the same array
+#pragma unroll
+    for (int k = 0; k < kOut; ++k) {
+      const int idx = tid + k * kDirectThreads;
+      gate_bits[kMats == 1 ? k : 0] = idx < n_out ? float_to_bf16_bits(total(0, idx)) : std::uint16_t{0};
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NCOL; ++n) red[0][n][warp][lane] = make_float4(acc2[n][0], acc2[n][1], acc2[n][2], acc2[n][3]);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int k = 0; k < kOut; ++k) {
+    const int idx = tid + k * kDirectThreads;
+    if (idx >= n_out) break;
     const int r = idx & 15, c = (idx >> 4) & 7, n = (idx >> 7) % NCOL, tile = (idx >> 7) / NCOL;
     const int row = (tile0 + tile) * 16 + r, col = 8 * n + c;
     if (col >= M || row >= N) continue;
-    const int src_lane = (r & 7) * 4 + (c >> 1);
-    const int elem = (r >> 3) * 2 + (c & 1);
-    const int w0 = tile * nsplit;
-    float v = 0.f;
-    for (int s = 0; s < nsplit; ++s) v += reinterpret_cast<const float*>(&red[0][n][w0 + s][src_lane])[elem];
-    std::uint16_t o = float_to_bf16_bits(v);
+    std::uint16_t o = (kMats == 1 && pair) ? gate_bits[kMats == 1 ? k : 0] : float_to_bf16_bits(total(0, idx));
     const std::size_t at = static_cast<std::size_t>(col) * N + row;
     if (pair) {
-      float u = 0.f;
-      for (int s = 0; s < nsplit; ++s) u += reinterpret_cast<const float*>(&red[1][n][w0 + s][src_lane])[elem];
       // CUDALM's rounding order (src/kernels/qwen35_kernels.cu:459-476)
-      o = silu_mul_bits(bf16_bits_to_float(o), float_to_bf16_bits(u));
+      o = silu_mul_bits(bf16_bits_to_float(o), float_to_bf16_bits(total(kMats - 1, idx)));
     } else if (mode == kDirectResidual) {
       o = add_bits(d.res[at], o);  // src/kernels/qwen35_kernels.cu:442-456
     }
@@ -328,7 +386,12 @@ int run_direct(const cudalm_b200_linear* ls, int count, const std::uint8_t* cons
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, mmax <= 8 ? w4a16_direct_kernel<1> : w4a16_direct_kernel<2>, p);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg,
+                                            mmax <= 8    ? w4a16_direct_kernel<1>
+                                            : mmax <= 16 ? w4a16_direct_kernel<2>
+                                            : mmax <= 32 ? w4a16_direct_kernel<4>
+                                                         : w4a16_direct_kernel<8>,
+                                            p);
   if (le != cudaSuccess) {
     g_last_cuda_error = static_cast<int>(le);
     (void)cudaGetLastError();

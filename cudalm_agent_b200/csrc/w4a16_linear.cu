@@ -381,10 +381,27 @@ int run_fallback(const cudalm_b200_linear& l, cudaStream_t stream) {
 // True when the lean kernel answers a single call: up to g_direct_max_bytes of weights, and
 // any number of bytes where K is beyond the streaming kernel's shared memory (K > 4096: the
 // other choice is the one-warp-per-row kernel; 8192 x 8192, one row: 65.6 -> 16.4 us).
+// From 17 to 64 rows it is the better one where a long K meets few weight rows (at most one
+// tile of 16 per SM): the tensor-memory kernels then walk K in a chain on few SMs.
 bool direct_takes(const cudalm_b200_linear& l, const std::uint8_t* weight2) {
   if (!direct_eligible(l, weight2)) return false;
   const long long limit = g_direct_max_bytes.load(std::memory_order_relaxed);
+  if (l.M > 16) {
+    if (l.K <= 2048 || (l.N + 15) / 16 > num_sms()) return false;
+    if (l.M < g_tc_min_rows.load(std::memory_order_relaxed)) return false;
+  }
   return direct_weight_bytes(l, weight2 != nullptr) <= limit || (limit > 0 && l.K > kMaxStreamK);
+}
+
+// Which of the tensor-memory kernels answers a single call of 17 rows and more.  Above 64
+// rows only the many-row kernel can.  From 33 it is faster on every shape (48 rows, many-row
+// kernel against the other, us: 512x1024 7.0 / 10.6, 6144x1024 7.2 / 11.3, 1024x3584 17.8 /
+// 19.1, 8192x8192 37.5 / 43.6, 32768x1024 13.7 / 14.2); with fewer rows the other one's read-back
+// is shorter and its split of a long K pays (17 rows: 512x1024 6.9 / 9.7, 1024x2048 11.0 / 13.3,
+// but 1024x3584 17.5 / 15.4, 8192x8192 37.3 / 35.3, 32768x1024 14.1 / 13.2).
+bool rows_take(const cudalm_b200_linear& l) {
+  if (l.M > 32) return true;
+  return l.M > 16 && l.K <= 2048 && static_cast<long long>(l.N) * (l.K / 2) <= (8ll << 20);
 }
 
 // One projection with any M: passes of as many rows as fit in shared memory.
@@ -392,9 +409,9 @@ int run_single(cudalm_b200_linear l, cudaStream_t stream) {
   if (int rc = validate(l)) return rc;
   if (direct_takes(l, nullptr)) return run_direct(&l, 1, nullptr, nullptr, nullptr, stream);
   if (l.M >= g_tc_min_rows.load(std::memory_order_relaxed)) {
-    // the tensor-memory kernels: one for up to 64 rows, one for any number above
+    // the tensor-memory kernels
+    if (rows_take(l) && rows_eligible(l)) return run_rows(&l, 1, nullptr, nullptr, nullptr, stream);
     if (l.M <= kTcMaxRows && tc_eligible(l)) return run_tc(&l, 1, stream);
-    if (l.M > kTcMaxRows && rows_eligible(l)) return run_rows(&l, 1, nullptr, nullptr, nullptr, stream);
   }
   if (!stream_eligible(l)) return run_fallback(l, stream);
   const int per_pass = max_rows_per_pass(l.K);
@@ -432,7 +449,8 @@ int run_extra(cudalm_b200_linear l, const LinearExtra& ex, cudaStream_t stream) 
   if (l.M >= g_tc_min_rows.load(std::memory_order_relaxed)) {
     // the tensor-memory kernels, when they take the call
     int rc = CUDALM_B200_ERR_UNSUPPORTED;
-    if (l.M > kTcMaxRows)
+    // (to 64 rows, outputs that the TMA unit cannot address stay with the streaming kernel)
+    if (rows_take(l) && (l.M > kTcMaxRows || (l.N % 8 == 0 && aligned_to(l.y, 16))))
       rc = run_rows(&l, 1, ex.weight2, ex.scales2, ex.residual, stream);
     else if (tc_eligible(l))
       rc = run_tc_extra(l, ex.weight2, ex.scales2, ex.residual, stream);
@@ -560,19 +578,20 @@ int cudalm_b200_linear_multi(const cudalm_b200_linear* linears, int count, void*
     bool all_direct = true;
     long long wbytes = 0;
     for (int i = 0; i < count; ++i) {
-      all_direct &= direct_eligible(linears[i], nullptr);
+      all_direct &= direct_eligible(linears[i], nullptr) && linears[i].M <= 16;
       wbytes += direct_weight_bytes(linears[i], false);
     }
     if (all_direct && wbytes <= g_direct_max_bytes.load(std::memory_order_relaxed))
       return run_direct(linears, count, nullptr, nullptr, nullptr, st);
   }
   if (mmax >= g_tc_min_rows.load(std::memory_order_relaxed)) {
-    bool all_tc = true;
-    for (int i = 0; i < count; ++i) all_tc &= tc_eligible(linears[i]);
-    if (all_tc) return run_tc(linears, count, st);
-    bool all_rows = mmax > kTcMaxRows;
-    for (int i = 0; i < count; ++i) all_rows &= rows_eligible(linears[i]);
+    bool all_rows = true, all_tc = true;
+    for (int i = 0; i < count; ++i) {
+      all_rows &= rows_eligible(linears[i]) && (mmax > kTcMaxRows || rows_take(linears[i]));
+      all_tc &= tc_eligible(linears[i]);
+    }
     if (all_rows) return run_rows(linears, count, nullptr, nullptr, nullptr, st);
+    if (all_tc) return run_tc(linears, count, st);
   }
   Plan pl;
   if (!all_stream || mmax > CUDALM_B200_MAX_GROUP_M || !make_plan(kmax, mmax, &pl)) {
@@ -663,6 +682,18 @@ int cudalm_b200_group_create(const cudalm_b200_linear* linears, int count,
     Plan probe;
     const bool stream_fits = m_all <= CUDALM_B200_MAX_GROUP_M && k_all <= kMaxStreamK &&
                              make_plan(k_all, m_all, &probe);
+    // a group of one runs as its single call does where that takes another kernel
+    const bool as_single = count == 1 && m_all > 16 && m_all >= g_tc_min_rows.load(std::memory_order_relaxed) &&
+                           linears[0].reserved == 0 &&
+                           (direct_takes(linears[0], nullptr) || (rows_take(linears[0]) && rows_eligible(linears[0])));
+    if (as_single) {
+      cudalm_b200_group* g = new cudalm_b200_group();
+      g->count = 1;
+      g->singles.assign(linears, linears + 1);
+      g->bytes = tc_bytes;
+      *group_out = g;
+      return CUDALM_B200_OK;
+    }
     if (m_all >= g_tc_min_rows.load(std::memory_order_relaxed) || !stream_fits) {
       TcGroup* tg = nullptr;
       const int rc = tc_group_create(linears, count, &tg);
