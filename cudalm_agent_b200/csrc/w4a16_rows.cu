@@ -189,17 +189,21 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
-// bf16(silu(gate)) of a bf16 value, the bits of silu_bits(): the approximate quotient (within
-// two units of the last of 24 bits; the denominator is kept inside its range) decides unless
-// it lies next to a rounding boundary of bf16, i.e. for all but one in 4,000 values.  The
-// correctly rounded division takes several times as long and was most of a pair's epilogue.
-__device__ __forceinline__ std::uint16_t silu_bits_near(std::uint16_t gate_bits) {
+// bf16(silu(gate)) of a bf16 value, the bits of silu_bits(): the quotient comes from an
+// approximate reciprocal and one Newton correction of its residual (Markstein's method)
+// without a branch.  Every bf16 argument was compared.  A denominator too large for its
+// reciprocal is scaled down; where the residual is not a number (an infinite gate or
+// denominator) the product stands.  A branch to the correctly rounded division, as rarely as
+// it was taken, cost 13 us of 69 (3584 x 1024, 2048 rows): its eight copies in the loop below.
+__device__ __forceinline__ std::uint16_t silu_bits_fast(std::uint16_t gate_bits) {
   const float g = bf16_bits_to_float(gate_bits);
-  const float d = 1.0f + expf(-g);
-  const float q = __fdividef(g, d);
-  const int off = static_cast<int>(__float_as_uint(q) & 0xFFFFu) - 0x8000;
-  if (d < 1e30f && (off > 8 || off < -8)) return float_to_bf16_bits(q);
-  return silu_bits(gate_bits);
+  const float scale = g < -64.f ? 0x1p-64f : 1.f;
+  const float d = (1.0f + expf(-g)) * scale;
+  float rc;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(d));
+  const float q = g * rc;
+  const float r = fmaf(-q, d, g);
+  return float_to_bf16_bits((r == r ? fmaf(r, rc, q) : q) * scale);
 }
 
 // The weight and activation tile of consecutive units of one projection.
@@ -581,7 +585,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               // CUDALM's rounding order: bf16 after each projection, after silu, after the product
-              const float silu = bf16_bits_to_float(silu_bits_near(static_cast<std::uint16_t>(w[k])));
+              const float silu = bf16_bits_to_float(silu_bits_fast(static_cast<std::uint16_t>(w[k])));
               *reinterpret_cast<std::uint16_t*>(slot16 + (i + k) * 64) =
                   float_to_bf16_bits(silu * bf16_bits_to_float(static_cast<std::uint16_t>(w[k] >> 16)));
             }

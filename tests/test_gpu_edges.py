@@ -225,9 +225,8 @@ def test_bound_calls_take_and_refuse_what_the_checks_do(eng):
 
 
 def test_many_row_silu_on_every_bf16_value(eng, orc):
-    """The many-row kernel's silu decides by an approximate quotient unless that lies next to
-    a rounding boundary: every bf16 gate value gives the bits of the lean kernel, which
-    divides with correct rounding."""
+    """The many-row kernel's silu corrects an approximate quotient: every bf16 gate value gives
+    the bits of the lean kernel, which divides with correct rounding."""
     import torch
     W = np.zeros((8, 64), np.uint8)
     W[:, 0] = 0x01                       # the gate output is x[0] ...
