@@ -216,14 +216,14 @@ def device_status() -> int:
 
 
 def set_tensor_path_min_rows(min_rows: int) -> int:
-    """Batched calls with at least this many rows take the tcgen05 kernel
+    """Batched calls with at least this many rows take the tcgen05 kernels
     (default 17); returns the previous value."""
     return int(load_library().cudalm_b200_set_tensor_path_min_rows(int(min_rows)))
 
 
 def set_direct_path_max_bytes(max_bytes: int) -> int:
-    """Single calls with at most 8 rows and at most this many weight bytes take
-    the lean kernel (0: never); returns the previous value."""
+    """Single calls with at most 16 rows (few weight rows: 64) and at most this many weight
+    bytes take the lean kernel (0: never); returns the previous value."""
     return int(load_library().cudalm_b200_set_direct_path_max_bytes(int(max_bytes)))
 
 

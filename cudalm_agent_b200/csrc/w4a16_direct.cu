@@ -137,7 +137,7 @@ __device__ __forceinline__ void direct_group(const uint4& qa, const uint4& qb,
     for (int i = 0; i < 4; ++i) sum[n][i] = c0[n][i] + c1[n][i];
 }
 
-// The same for four or eight column tiles: the activations of one weight word at a time, the
+// The same for four to eight column tiles: the activations of one weight word at a time, the
 // next word's requested before this one's MMAs.
 template <int NCOL>
 __device__ __forceinline__ void direct_group_wide(const uint4& qa, const uint4& qb,
@@ -390,6 +390,7 @@ int run_direct(const cudalm_b200_linear* ls, int count, const std::uint8_t* cons
                                             mmax <= 8    ? w4a16_direct_kernel<1>
                                             : mmax <= 16 ? w4a16_direct_kernel<2>
                                             : mmax <= 32 ? w4a16_direct_kernel<4>
+                                            : mmax <= 48 ? w4a16_direct_kernel<6>
                                                          : w4a16_direct_kernel<8>,
                                             p);
   if (le != cudaSuccess) {

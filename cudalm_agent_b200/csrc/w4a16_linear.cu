@@ -382,12 +382,16 @@ int run_fallback(const cudalm_b200_linear& l, cudaStream_t stream) {
 // any number of bytes where K is beyond the streaming kernel's shared memory (K > 4096: the
 // other choice is the one-warp-per-row kernel; 8192 x 8192, one row: 65.6 -> 16.4 us).
 // From 17 to 64 rows it is the better one where a long K meets few weight rows (at most one
-// tile of 16 per SM): the tensor-memory kernels then walk K in a chain on few SMs.
+// tile of 16 per SM): the tensor-memory kernels then walk K in a chain on few SMs (lean
+// against the other, us, 17 / 32 / 48 / 64 rows: 1024x3584 6.2 / 7.3 / 9.6 / 12.9 against
+// 15.8 / 16.1 / 17.8 / 17.8; 2368x2048 at 32 / 48 / 64: 5.6 / 6.9 / 9.2 against 11.4 / 11.6 /
+// 11.6).  It is faster on shorter K too, but a fused pair is not, and a pair is to give the
+// bits of its two projections.
 bool direct_takes(const cudalm_b200_linear& l, const std::uint8_t* weight2) {
   if (!direct_eligible(l, weight2)) return false;
   const long long limit = g_direct_max_bytes.load(std::memory_order_relaxed);
   if (l.M > 16) {
-    if (l.K <= 2048 || (l.N + 15) / 16 > num_sms()) return false;
+    if (l.K < 2048 || (l.N + 15) / 16 > num_sms()) return false;
     if (l.M < g_tc_min_rows.load(std::memory_order_relaxed)) return false;
   }
   return direct_weight_bytes(l, weight2 != nullptr) <= limit || (limit > 0 && l.K > kMaxStreamK);

@@ -27,7 +27,7 @@
 // 1024 and 2048 rows took 40 us instead of 29); so each role waits once per group on all it
 // needs, and one barrier per group tells everybody that its MMAs are done.  2048 rows of a
 // layer with hidden size 1024 (four calls): 2018 us as passes of 64 rows, 180 with direct
-// stores and three commits per group, 145 now.
+// stores and three commits per group, 128 now.
 //
 // Every wait is bounded; a wait that runs out raises a CTA-wide abort flag, the kernel
 // stores ERR_TIMEOUT in the status word, frees its tensor memory and returns.
@@ -565,8 +565,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) w4a16_rows_kernel(const __gri
           // An even lane holds the gate and its odd neighbour the up output of one row: they
           // exchange one of every two values, and each finishes one activation row.  The
           // box first takes {gate, up} words and is then rewritten from the front, eight
-          // words a lane at a time (all of a thread's values unrolled: 71.6 us against 68.8
-          // for 3584 x 1024 and 2048 rows).
+          // words a lane at a time (unrolled over all of them the code misses the
+          // instruction cache).
           std::uint32_t* words = reinterpret_cast<std::uint32_t*>(box) + lane;
 #pragma unroll
           for (int n = 0; n < kRowsChunk; n += 2) {
@@ -716,11 +716,11 @@ int run_rows(const cudalm_b200_linear* ls, int count, const std::uint8_t* weight
   // are its groups' and a fixed part (filling the pipeline, outputs).  Measured on 1024 x
   // 3584 and 6144 x 1024 with 2048 rows, 256 / 128 / 64: 29.3 / 19.8 / 34.4 and 29.4 / 34.9 /
   // 54.2 us.  A pair's silu lengthens the fixed part; with 128 sums a thread it has no
-  // registers (3584 x 1024, 2048 rows: 140 us against 70 and 78).
+  // registers (3584 x 1024, 2048 rows: 140 us against 55).
   static constexpr int kTiles[3] = {256, 128, 64};
   static constexpr int kPerGroup[3] = {1560, 1075, 965};
   static constexpr int kPerUnit[3] = {6000, 2400, 1600};
-  static constexpr int kPerPair[3] = {0, 10300, 3700};
+  static constexpr int kPerPair[3] = {0, 6300, 2800};
   int nt = 0;
   long long best = 0;
   for (int k = pair ? 1 : 0; k < 3; ++k) {

@@ -79,8 +79,10 @@ CUDALM_B200_API int cudalm_b200_int4_gemv_bf16(const uint8_t* weight, const uint
  * (CUDALM include/cudalm/kernels/batch_decode.h:61-63,
  *  src/kernels/batch_decode.cu:95-190,647-659): x is [B, K], y is [B, N].
  * Unlike CUDALM's, the weights are read once for all B rows.
- * From 17 rows on (tensor-memory kernel), a call whose projections have few rows
- * and K >= 2048 cuts K into slices that separate CTAs work on and adds them up in a
+ * From 17 rows on the tensor-memory kernels answer; above 64 rows one launch takes any
+ * number of them.  From 17 to 64 rows (where neither the many-row kernel nor, for at most
+ * one tile of 16 weight rows per SM and K >= 2048, the lean kernel is faster) a call whose projections
+ * have few rows and K >= 2048 cuts K into slices that separate CTAs work on and adds them up in a
  * fixed order in a second launch; the fp32 partial sums live in stream-ordered
  * scratch from a memory pool the library owns (allocated and freed on `stream`, so
  * the call stays asynchronous and can be captured in a CUDA graph).  The same holds
@@ -143,8 +145,9 @@ CUDALM_B200_API int cudalm_b200_gate_up_bf16(const uint8_t* gate_weight,
  * bf16 outputs of the gate and up projections of x [M, K]; replaces the two
  * projections and qwen35_silu_mul (CUDALM include/cudalm/kernels/qwen35_kernels.h:137-155,
  * src/kernels/qwen35_kernels.cu:459-476; call sites src/runtime/qwen35_deltanet.cpp:236-247,
- * src/runtime/qwen35_full_attention.cpp:317-331) with one launch per 16 rows, or per
- * 64 rows when M is at least the tensor path's smallest row count.
+ * src/runtime/qwen35_full_attention.cpp:317-331) with one launch per 16 rows, or one
+ * launch when M is at least the tensor path's smallest row count (to 64 rows: where N is a
+ * multiple of 8 and the output 16-byte aligned).
  * linear_residual: y[m][n] = bf16(float(residual[m][n]) + float(p)) with p the bf16
  * output of the projection; replaces the down / o_proj / out_proj projection and the
  * qwen35_add that follows it (src/kernels/qwen35_kernels.cu:442-456;
@@ -410,10 +413,12 @@ CUDALM_B200_API int cudalm_b200_quantize_w4a16(const uint16_t* w_bf16, int N, in
  * src/kernels/batch_decode.cu:95-190.) */
 CUDALM_B200_API int cudalm_b200_set_tensor_path_min_rows(int min_rows);
 /* Single calls (int4_gemv_bf16, batch_int4_gemv_bf16, linear_multi, gate_up*,
- * linear_residual) with at most 8 activation rows whose weights total at most
+ * linear_residual) with at most 16 activation rows whose weights total at most
  * max_bytes take the lean kernel, which has no set-up cost and answers a call of a
  * few megabytes in about one memory round trip; larger ones stream through the
- * persistent kernel.  0 switches the lean kernel off.  Returns the previous value.
+ * persistent kernel, unless K > 4096, which that one does not take.  From 17 to 64 rows
+ * single projections of at most one tile of 16 weight rows per SM and K >= 2048 take it
+ * too.  0 switches the lean kernel off.  Returns the previous value.
  * (CUDALM's counterpart is its one kernel per call,
  * src/kernels/int4_gemv_bf16.cu:221-243.) */
 CUDALM_B200_API int64_t cudalm_b200_set_direct_path_max_bytes(int64_t max_bytes);

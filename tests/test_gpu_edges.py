@@ -91,8 +91,15 @@ ROWS_SHAPES = [(304, 1024, 17), (1104, 2048, 40), (136, 384, 64), (1, 128, 65), 
                (19000, 128, 70), (40000, 128, 33)]
 
 
+@pytest.fixture
+def no_lean(eng):
+    prev = eng.set_direct_path_max_bytes(0)
+    yield
+    eng.set_direct_path_max_bytes(prev)
+
+
 @pytest.mark.parametrize("N,K,M", ROWS_SHAPES)
-def test_many_rows(eng, orc, N, K, M):
+def test_many_rows(eng, orc, no_lean, N, K, M):
     """Plain, residual (also in place) and gate/up forms of many rows against the oracle,
     and twice for equal bits; outputs off 16 bytes and off the matrix stay untouched."""
     import torch
@@ -141,9 +148,10 @@ def test_many_rows_in_one_call_with_few(eng, orc):
 
 @pytest.mark.parametrize("N,K,M", [(1, 128, 9), (17, 384, 16), (40, 1152, 10), (5003, 2944, 13), (1000, 1024, 15),
                                    (33, 4224, 1), (100, 8192, 8), (257, 8320, 16), (15, 16384, 9), (700, 4096, 12),
-                                   (100, 4224, 17), (257, 2176, 33), (2368, 2176, 64), (17, 8192, 40), (1024, 3584, 32)])
+                                   (100, 4224, 17), (257, 2176, 33), (2368, 2176, 64), (17, 8192, 40), (1024, 3584, 32),
+                                   (512, 2048, 48), (2368, 2048, 49), (1, 2176, 64)])
 def test_lean_kernel_on_more_rows_and_any_k(eng, orc, N, K, M):
-    """One, two, four and eight column tiles, K splits of equal and unequal length, K beyond the
+    """One, two, four, six and eight column tiles, K splits of equal and unequal length, K beyond the
     streaming kernel's limit: plain, residual and gate/up forms against the oracle."""
     import torch
     W, S = raw_weights(N, K, BASE_SEED + N)
