@@ -23,8 +23,15 @@
 //     MMAs per group and tile, then acc += scale * group_sum in fp32.  Products are exact,
 //     sums are fp32, activations are used as they are (any finite or non-finite
 //     value), and a group of zero nibbles contributes an exact zero;
-//   * the warps' partial sums meet in 4 KB of shared memory and are added in the
-//     fixed order of the K splits, so results do not depend on timing.
+//   * the warps' partial sums meet in shared memory (4 KB per tile of 8 activation rows and
+//     matrix) and are added in the fixed order of the K splits, so results do not depend
+//     on timing.
+//
+// What bounds it: one or two DRAM round trips, and with many activation rows their reads,
+// which every tile of 16 weight rows repeats from L2 (5003 x 2944: 4.5 us with one row, 8.0
+// with 9, 10.5 with 16; the streaming kernel, which stages them in every CTA, 8.4, 23.6 and
+// 26.1).  Where K > 4096 the streaming kernel's stages do not fit: 8192 x 8192 took 65.6 us
+// with one warp per row and takes 16.4 here.
 //
 // The MLP epilogues of the streaming kernel are available here too: a pair
 // (out = silu(gate x) * (up x): every warp works on its K split of both matrices,

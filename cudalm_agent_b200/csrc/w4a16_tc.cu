@@ -1,4 +1,6 @@
-// Batched rows (M >= 17 by default) on the fifth-generation tensor cores.
+// Batched rows (M >= 17 by default, at most 64) on the fifth-generation tensor cores:
+// grouped launches, the vocabulary projection, and single calls of 17 to 32 rows with a long
+// or large weight matrix (the many-row kernel, w4a16_rows.cu, answers the others).
 //
 // One CTA per SM works on items of 256 weight rows (two 128-row MMA tiles) of one
 // projection; the M activation rows (padded to NTOK = 16, 32 or 64) are the N
@@ -1099,7 +1101,8 @@ int tc_run_params(TcParams& p, int ntok, cudaStream_t stream, int* grid_out = nu
 
 // One projection with an MLP epilogue: weight2/scales2 non-null -> out = silu(W x) * (W2 x),
 // residual non-null -> out = residual + W x.  UNSUPPORTED unless the outputs can take
-// the TMA store and the second matrix is 16-byte aligned.
+// the TMA store and the second matrix is 16-byte aligned, and above 32 rows (the many-row
+// kernel's).
 int run_tc_extra(const cudalm_b200_linear& l, const std::uint8_t* weight2,
                  const std::uint16_t* scales2, const std::uint16_t* residual, cudaStream_t stream) {
   TcParams p;
@@ -1107,6 +1110,7 @@ int run_tc_extra(const cudalm_b200_linear& l, const std::uint8_t* weight2,
   int ntok = 0;
   TcScratchPlan plan;
   if (weight2 && (!aligned_to(weight2, 16) || !scales2)) return CUDALM_B200_ERR_UNSUPPORTED;
+  if (l.M > 32) return CUDALM_B200_ERR_UNSUPPORTED;
   if (int rc = tc_describe(&l, 1, p.inl, &p.total_items, &p.total_cost, &ntok, &plan, weight2 != nullptr))
     return rc;
   TcDesc& d = p.inl[0];
@@ -1126,9 +1130,7 @@ int run_tc_extra(const cudalm_b200_linear& l, const std::uint8_t* weight2,
   p.n_desc = 1;
   p.status = device_status_word();
   if (!p.status) return CUDALM_B200_ERR_CUDA;
-  const int rc = ntok == 16   ? tc_launch<16, true>(p, stream)
-                 : ntok == 32 ? tc_launch<32, true>(p, stream)
-                              : tc_launch<64, true>(p, stream);
+  const int rc = ntok == 16 ? tc_launch<16, true>(p, stream) : tc_launch<32, true>(p, stream);
   if (rc != CUDALM_B200_OK) return rc;
   return tc_launch_combine(p, ntok, plan.tiles, stream);
 }
